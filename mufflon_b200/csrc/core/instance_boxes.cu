@@ -98,7 +98,26 @@ __global__ void k_tight_boxes(const DLod* lods, const uint32_t* instLod, const f
 	}
 }
 
+__global__ void k_instance_records(const DLod* lods, const uint32_t* instLod, const float4* w2i, uint32_t n, InstRec* out) {
+	const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+	if(i >= n) return;
+	const uint32_t li = instLod[i];
+	InstRec r;
+	r.r0 = w2i[3 * size_t(i)]; r.r1 = w2i[3 * size_t(i) + 1]; r.r2 = w2i[3 * size_t(i) + 2];
+	r.nodes = nullptr; r.soup = nullptr; r.numPrims = 0;
+	r.pad[0] = r.pad[1] = r.pad[2] = 0;
+	if(li != 0xFFFFFFFFu) { r.nodes = lods[li].wnodes; r.soup = lods[li].wsoup; r.numPrims = lods[li].numPrims; }
+	out[i] = r;
+}
+
 } // namespace
+
+cudaError_t instance_records(const DLod* lods, const uint32_t* instLod, const float4* w2i, uint32_t n, InstRec* out,
+                             cudaStream_t stream) {
+	if(n == 0) return cudaSuccess;
+	k_instance_records<<<(n + 127) / 128, 128, 0, stream>>>(lods, instLod, w2i, n, out);
+	return cudaGetLastError();
+}
 
 cudaError_t tight_instance_boxes(const DLod* lods, const uint32_t* instLod, const float* instToWorld, uint32_t n,
                                  const float* looseBoxes, float* out, cudaStream_t stream) {

@@ -16,4 +16,8 @@ namespace mb {
 cudaError_t tight_instance_boxes(const DLod* lods, const uint32_t* instLod, const float* instToWorld, uint32_t n,
                                  const float* looseBoxes, float* out, cudaStream_t stream);
 
+// out[i] = what a ray needs to enter instance i (masked instances: no object).
+cudaError_t instance_records(const DLod* lods, const uint32_t* instLod, const float4* w2i, uint32_t n, InstRec* out,
+                             cudaStream_t stream);
+
 } // namespace mb

@@ -158,13 +158,13 @@ void DeviceScene::release() {
 	for(auto& l : lods) l.release();
 	lods.clear();
 	lodSources.clear();
-	cudaFree(dLods); cudaFree(dW2I); cudaFree(dInstLod); cudaFree(dInstBoxes); cudaFree(dInstCentroids);
+	cudaFree(dLods); cudaFree(dW2I); cudaFree(dInstLod); cudaFree(dInstRecs); cudaFree(dInstBoxes); cudaFree(dInstCentroids);
 	tlas.release();
 	cudaFree(dMaterials);
 	for(auto* t : textureBuffers) cudaFree(t);
 	textureBuffers.clear();
 	cudaFree(dTextures); cudaFree(dLights); cudaFree(dLightNodes); cudaFree(dLightKeys); cudaFree(dLightCodes);
-	dLods = nullptr; dW2I = nullptr; dInstLod = nullptr; dInstBoxes = nullptr; dInstCentroids = nullptr;
+	dLods = nullptr; dW2I = nullptr; dInstLod = nullptr; dInstRecs = nullptr; dInstBoxes = nullptr; dInstCentroids = nullptr;
 	dMaterials = nullptr; dTextures = nullptr; dLights = nullptr; dLightNodes = nullptr;
 	dLightKeys = nullptr; dLightCodes = nullptr;
 	cudaFree(dInstI2W); cudaFree(dWideInstBoxes); cudaFree(dLightMirror); cudaFree(dLightFirst); cudaFree(dLightLods);
@@ -356,6 +356,11 @@ bool build_device_scene(MufflonInstance& inst, std::string& err) {
 	if(!upload(D.dInstBoxes, D.cap[3], boxes.data(), size_t(numInst) * 6, s, err)) return false;
 	if(!upload(D.dInstCentroids, D.cap[4], cents.data(), size_t(numInst) * 3, s, err)) return false;
 	if(!upload(D.dInstI2W, D.lightCap[0], i2wAll.data(), size_t(numInst) * 12, s, err)) return false;
+	if(!reserve_device(D.dInstRecs, D.cap[12], numInst, err)) return false;
+	{
+		const cudaError_t e = instance_records(D.dLods, D.dInstLod, D.dW2I, numInst, D.dInstRecs, s);
+		if(e != cudaSuccess) { err = std::string("instance records failed: ") + cudaGetErrorString(e); return false; }
+	}
 	if(active > 1) {
 		SceneBuildInput sin{};
 		sin.numInstances = numInst; sin.activeInstances = uint32_t(active);
@@ -474,7 +479,7 @@ bool build_device_scene(MufflonInstance& inst, std::string& err) {
 	DScene& S = D.desc;
 	S = DScene{};
 	S.lods = D.dLods; S.numLods = uint32_t(D.lods.size());
-	S.worldToInstance = D.dW2I; S.instanceLod = D.dInstLod; S.numInstances = numInst;
+	S.worldToInstance = D.dW2I; S.instanceLod = D.dInstLod; S.instRecs = D.dInstRecs; S.numInstances = numInst;
 	S.activeInstances = active; S.validInstance = valid;
 	S.maxSteps = MAX_TRAVERSAL_STEPS;
 	S.hasAlpha = hasAlpha ? 1 : 0;

@@ -161,6 +161,7 @@ struct DeviceScene {
 	DLod* dLods = nullptr;
 	float4* dW2I = nullptr;
 	uint32_t* dInstLod = nullptr;
+	InstRec* dInstRecs = nullptr;
 	float* dInstBoxes = nullptr;
 	float* dInstCentroids = nullptr;
 	BvhBuffers tlas;
@@ -188,7 +189,7 @@ struct DeviceScene {
 	DScene desc{};
 	float aabb[6] = { 0, 0, 0, 0, 0, 0 };
 	bool valid = false;
-	size_t cap[12] = {};
+	size_t cap[13] = {};
 	// host-side times of the last load (ms) and its host-to-device bytes
 	float loadMs[5] = {};          // total, geometry upload, object BVHs, instance BVH, lights/materials
 	uint64_t loadH2dBytes = 0;

@@ -451,8 +451,8 @@ __global__ void k_soup(LodBuildInput in, int n, const int32_t* __restrict__ prim
 }
 
 // Soup of the wide hierarchy's primitive order: slot k holds primitive
-// wprims[k]; for triangles the three vertices, and the primitive id in the
-// w component of the first float4 for every primitive type.
+// wprims[k]; for triangles the three vertices, and for every primitive type
+// its id in the first row's w and its kind in the second's.
 __global__ void k_wsoup(LodBuildInput in, int n, const int32_t* __restrict__ wprims, float4* soup) {
 	const int k = blockIdx.x * blockDim.x + threadIdx.x;
 	if(k >= n) return;
@@ -462,7 +462,7 @@ __global__ void k_wsoup(LodBuildInput in, int n, const int32_t* __restrict__ wpr
 		const uint32_t t = uint32_t(p) * 3;
 		const f3 v0 = v3(in.vertices, in.indices[t]), v1 = v3(in.vertices, in.indices[t + 1]), v2 = v3(in.vertices, in.indices[t + 2]);
 		a = make_float4(v0.x, v0.y, v0.z, __int_as_float(p));
-		b = make_float4(v1.x, v1.y, v1.z, 0.0f);
+		b = make_float4(v1.x, v1.y, v1.z, __int_as_float(SOUP_TRIANGLE));
 		c = make_float4(v2.x, v2.y, v2.z, 0.0f);
 	}
 	soup[3 * size_t(k)] = a;

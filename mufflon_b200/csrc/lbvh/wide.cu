@@ -179,12 +179,13 @@ __global__ void __launch_bounds__(128) k_wide_level(WideBuildArgs A, const int2*
 			}
 			if(inner[i]) {
 				imask |= 1u << s;
+				meta[s >> 2] |= uint32_t((1 << 5) | (24 + s)) << (8 * (s & 3));
 				const uint32_t q = queueBase + uint32_t(innerRank);
 				const uint32_t idx = childBase + uint32_t(innerRank++);
 				if(q < A.nodeCapacity) qout[q] = make_int2(ch[i], int(idx));
 				else bad = true;
 			} else {
-				meta[s >> 2] |= uint32_t((cnt[i] << 5) | primOffset) << (8 * (s & 3));
+				meta[s >> 2] |= uint32_t((((1 << cnt[i]) - 1) << 5) | primOffset) << (8 * (s & 3));
 				for(int j = 0; j < cnt[i]; ++j) A.prims[primBase + uint32_t(primOffset + j)] = A.sortedIds[first[i] + j];
 				primOffset += cnt[i];
 			}

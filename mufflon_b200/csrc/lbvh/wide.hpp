@@ -17,8 +17,11 @@
 //     box that contains a hit point (the step is far larger than the rounding
 //     error of that expression);
 //   * leaves hold at most WIDE_LEAF_MAX primitives of one contiguous range;
-//     meta[slot] = (count << 5) | offset, offset relative to the node's
-//     primitive base, so a node's hit leaves become one 32-bit primitive mask.
+//     meta[slot] = (one bit per primitive << 5) | offset, offset relative to
+//     the node's primitive base, and (1 << 5) | (24 + slot) for an internal
+//     child: shifting the upper three bits by the lower five and or-ing the
+//     hit slots gives the node's hit primitives in bits 0-23 and its hit
+//     internal children in bits 24-31 of one word.
 #pragma once
 
 #include <cstdint>
@@ -29,12 +32,16 @@ namespace mb {
 constexpr int WIDE_LEAF_MAX = 3;       // primitives per leaf in object hierarchies
 constexpr int WIDE_TLAS_LEAF_MAX = 1;  // instances per leaf in the instance hierarchy
 
+// In the second row's w of a primitive's soup: its kind, so that the traversal
+// needs no primitive counts of the object.
+constexpr int SOUP_TRIANGLE = 1;
+
 struct alignas(16) WideNode {
 	float p[3];            // grid origin
 	uint32_t eimask;       // biased exponents ex | ey << 8 | ez << 16, internal-slot mask << 24
 	uint32_t childBase;    // index of the first internal child
 	uint32_t primBase;     // first slot of this node's leaf primitives
-	uint32_t meta[2];      // per slot (count << 5) | offset, 0 for internal / empty slots
+	uint32_t meta[2];      // per slot (unary count << 5) | offset, (1 << 5) | (24 + slot) internal, 0 empty
 	uint32_t qlo[3][2];    // per axis, 8 slots of 8 bits
 	uint32_t qhi[3][2];
 };

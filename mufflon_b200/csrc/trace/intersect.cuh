@@ -40,20 +40,24 @@ MBD float slab_rcp(float x) {
 	return fminf(fmaxf(__fdiv_rn(1.0f, x), -18446744073709551616.0f), 18446744073709551616.0f);
 }
 
+// Axes and shear constants of the watertight triangle test for direction d.
+MBD void shear(f3 d, int& kx, int& ky, int& kz, float& Sx, float& Sy, float& Sz) {
+	const float ax = fabsf(d.x), ay = fabsf(d.y), az = fabsf(d.z);
+	kz = (ax >= ay && ax >= az) ? 0 : (ay >= az ? 1 : 2);
+	kx = kz + 1 == 3 ? 0 : kz + 1;
+	ky = kx + 1 == 3 ? 0 : kx + 1;
+	if(d[kz] < 0.0f) { const int t = kx; kx = ky; ky = t; }
+	Sx = __fdiv_rn(d[kx], d[kz]);
+	Sy = __fdiv_rn(d[ky], d[kz]);
+	Sz = __fdiv_rn(1.0f, d[kz]);
+}
+
 MBD FastRay make_ray(f3 o, f3 d) {
 	FastRay r;
 	r.o = o;
 	r.d = d;
 	r.inv = make3(slab_rcp(d.x), slab_rcp(d.y), slab_rcp(d.z));
-	const float ax = fabsf(d.x), ay = fabsf(d.y), az = fabsf(d.z);
-	int kz = (ax >= ay && ax >= az) ? 0 : (ay >= az ? 1 : 2);
-	int kx = kz + 1 == 3 ? 0 : kz + 1;
-	int ky = kx + 1 == 3 ? 0 : kx + 1;
-	if(d[kz] < 0.0f) { const int t = kx; kx = ky; ky = t; }
-	r.kx = kx; r.ky = ky; r.kz = kz;
-	r.Sx = __fdiv_rn(d[kx], d[kz]);
-	r.Sy = __fdiv_rn(d[ky], d[kz]);
-	r.Sz = __fdiv_rn(1.0f, d[kz]);
+	shear(d, r.kx, r.ky, r.kz, r.Sx, r.Sy, r.Sz);
 	return r;
 }
 
@@ -86,14 +90,14 @@ static __device__ __noinline__ float3 edge_functions_double(float Ax, float Ay, 
 }
 
 // Watertight ray/triangle test (Woop, Benthin, Wald, JCGT 2013).
-MBD bool tri_test(const FastRay& r, f3 v0, f3 v1, f3 v2, float& t, f2& bary) {
-	const f3 A = v0 - r.o, B = v1 - r.o, C = v2 - r.o;
-	const float Ax = A[r.kx] - r.Sx * A[r.kz];
-	const float Ay = A[r.ky] - r.Sy * A[r.kz];
-	const float Bx = B[r.kx] - r.Sx * B[r.kz];
-	const float By = B[r.ky] - r.Sy * B[r.kz];
-	const float Cx = C[r.kx] - r.Sx * C[r.kz];
-	const float Cy = C[r.ky] - r.Sy * C[r.kz];
+MBD bool tri_test(f3 o, int kx, int ky, int kz, float Sx, float Sy, float Sz, f3 v0, f3 v1, f3 v2, float& t, f2& bary) {
+	const f3 A = v0 - o, B = v1 - o, C = v2 - o;
+	const float Ax = A[kx] - Sx * A[kz];
+	const float Ay = A[ky] - Sy * A[kz];
+	const float Bx = B[kx] - Sx * B[kz];
+	const float By = B[ky] - Sy * B[kz];
+	const float Cx = C[kx] - Sx * C[kz];
+	const float Cy = C[ky] - Sy * C[kz];
 	float U = Cx * By - Cy * Bx;
 	float V = Ax * Cy - Ay * Cx;
 	float W = Bx * Ay - By * Ax;
@@ -104,13 +108,16 @@ MBD bool tri_test(const FastRay& r, f3 v0, f3 v1, f3 v2, float& t, f2& bary) {
 	if((U < 0.0f || V < 0.0f || W < 0.0f) && (U > 0.0f || V > 0.0f || W > 0.0f)) return false;
 	const float det = U + V + W;
 	if(det == 0.0f) return false;
-	const float Az = r.Sz * A[r.kz];
-	const float Bz = r.Sz * B[r.kz];
-	const float Cz = r.Sz * C[r.kz];
+	const float Az = Sz * A[kz];
+	const float Bz = Sz * B[kz];
+	const float Cz = Sz * C[kz];
 	const float T = U * Az + V * Bz + W * Cz;
 	t = __fdiv_rn(T, det);
 	bary = make2(__fdiv_rn(U, det), __fdiv_rn(V, det));
 	return true;
+}
+MBD bool tri_test(const FastRay& r, f3 v0, f3 v1, f3 v2, float& t, f2& bary) {
+	return tri_test(r.o, r.kx, r.ky, r.kz, r.Sx, r.Sy, r.Sz, v0, v1, v2, t, bary);
 }
 
 MBD bool solve_square(float a, float b, float c, float& x0, float& x1) {

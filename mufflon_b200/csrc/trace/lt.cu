@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(128, 6) k_lt(const DScene S, const LtParams P,
 			t.init(S, ro, rd, tmax, shadow, cnt);
 			while(!t.step(S, cnt, stack)) {}
 			if(shadow) {
-				if(!t.occluded) {
+				if(!t.occluded()) {
 					atomicAdd(T.iter + pix, add);
 					if(T.density) atomicAdd(T.iterDensity + pix, dens);
 					if(T.recPixel) {
@@ -225,11 +225,11 @@ __global__ void __launch_bounds__(128, 6) k_lt(const DScene S, const LtParams P,
 						o[0] = add.x; o[1] = add.y; o[2] = add.z; o[3] = add.w; o[4] = dens;
 					}
 				}
-			} else if(!t.best.has) {
+			} else if(!t.hit().has) {
 				T.rngState[ph.photon] = ph.rng;
 				phase = PH_IDLE;
 			} else {
-				const Intersection hit = hit_attributes(S, ro, rd, t.best);
+				const Intersection hit = hit_attributes(S, ro, rd, t.hit());
 				ph.position = ro + rd * hit.distance;
 				ph.ts = tangent_space(S, hit);
 				ph.mat = fetch_material(S, material_index(S, hit.inst, hit.prim), hit.uv);

@@ -76,11 +76,11 @@ MBD void trace_ray_queue(const DScene& S, const RayQueue& Q, TraceCounters* coun
 		if(active && t.step(S, cnt, stack)) {
 			active = false;
 			if(item < Q.nExt) {
-				const HitRec& h = t.best;
+				const HitRec h = t.hit();
 				__stcs(Q.hit + item, make_float4(h.t, __int_as_float(h.has ? h.inst : -1), __int_as_float(h.has ? h.prim : -1), h.sp.x));
 				__stcs(Q.hitV + item, h.sp.y);
 			} else {
-				visible(item - Q.nExt, t.occluded);
+				visible(item - Q.nExt, t.occluded());
 			}
 		}
 	}

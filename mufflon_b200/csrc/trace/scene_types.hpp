@@ -51,6 +51,17 @@ struct DLod {
 	int32_t numWide;
 };
 
+// What a ray needs to enter an instance, in one place: the world-to-instance
+// rows and the object's traversal hierarchy (entering read instance, object
+// index and object record one after the other before).
+struct alignas(16) InstRec {
+	float4 r0, r1, r2;
+	const WideNode* nodes;
+	const float4* soup;
+	int32_t numPrims, pad[3];
+};
+static_assert(sizeof(InstRec) == 80, "InstRec layout");
+
 struct DMaterial {
 	int32_t type;
 	float albedo[3];
@@ -102,6 +113,7 @@ struct DScene {
 	uint32_t numLods;
 	const float4* worldToInstance; // 3 float4 (rows) per instance
 	const uint32_t* instanceLod;
+	const InstRec* instRecs;       // per instance (masked ones unset)
 	uint32_t numInstances;
 	int32_t activeInstances;
 	uint32_t validInstance;

@@ -388,14 +388,14 @@ __global__ void __launch_bounds__(128, MINB) k_trace(const SP sp, WfState W, int
 		if(active && t.step(sp.scene(path), cnt, stack)) {
 			if(item < nExt) {
 				stats_add(stats, 0, cnt);
-				const HitRec& h = t.best;
+				const HitRec h = t.hit();
 				__stcs(W.qHit[q] + ent, make_float4(h.t, __int_as_float(h.has ? h.inst : -1), __int_as_float(h.has ? h.prim : -1), h.sp.x));
 				__stcs(W.qHitSpy[q] + ent, h.sp.y);
 				active = false;
 			} else {
 				stats_add(stats, 1, cnt);
 				const unsigned slot = ent * unsigned(neeCount) + unsigned(ray);
-				if(!t.occluded) {
+				if(!t.occluded()) {
 					const float4 c4 = __ldcs(W.sContrib + slot);
 					const f3 c = f4to3(c4);
 					radiance = contribute(radiance, c);
@@ -821,7 +821,7 @@ __global__ void __launch_bounds__(128, MINB) k_tail(const SP sp, WfState W, int 
 		while(!t.step(S, cnt, stack)) {}
 		stats_add(stats, shadow ? 1 : 0, cnt);
 		if(shadow) {
-			if(!t.occluded) {
+			if(!t.occluded()) {
 				radiance = contribute(radiance, c);
 				if constexpr(SP::adjoint) {
 					const f3 cc = contribute(make3(0.0f, 0.0f, 0.0f), c);
@@ -836,7 +836,7 @@ __global__ void __launch_bounds__(128, MINB) k_tail(const SP sp, WfState W, int 
 			++i;
 		} else {
 			++b;
-			begin_vertex(ro, rd, t.best, v.position);
+			begin_vertex(ro, rd, t.hit(), v.position);
 		}
 	}
 	__syncthreads();

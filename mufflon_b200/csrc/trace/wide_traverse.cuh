@@ -5,8 +5,8 @@
 // One loop runs both levels. The state of a ray is
 //   * a node group: the child base of the last visited node, its internal-slot
 //     mask and the still unvisited hit internal children as bits in
-//     traversal order (bit k = slot k ^ flip, flip chosen from the ray's
-//     direction octant so that bit order is roughly near to far),
+//     traversal order (bit 24 + (slot ^ octant of the ray's direction), so
+//     that the highest bit is roughly the nearest child),
 //   * a primitive group: the last visited node's primitive base and one bit
 //     per primitive of its hit leaves,
 //   * a stack of node groups (and, at the instance level, primitive groups of
@@ -15,6 +15,18 @@
 // stack depth; when the object level's groups are exhausted at that depth the
 // world ray is restored. Every step visits one node (eight box tests that do
 // the same arithmetic in every lane) and then that node's hit primitives.
+//
+// What bounds it: divergence and instruction issue (ncu, incoherent bounce of
+// the 1080p icosphere: 7.5 of 32 lanes per instruction, 575 warp instructions
+// per ray, memory below 10 % of its peak), so the step is written for few
+// instructions and registers: box planes from biased bytes in packed
+// multiply-adds, hit masks by shifts of precomputed bytes, approximate
+// reciprocals for boxes, one record per instance, no world-ray shear
+// constants, entering an instance in the step that visits its root. Against
+// an IEEE-reciprocal form with a subtraction per plane byte, out-of-line
+// instance transforms and the prepared world ray in registers (same box, per
+// iteration): trace stage of the 1080p icosphere 2.90 -> 2.12 ms, of 4 096
+// instances at 720p 15.4 -> 14.3 ms; spilled bytes at 80 registers 360 -> 204.
 //
 // The box test cannot cull a box that contains a hit point (wide.hpp), so the
 // closest hit is the minimum of (world t, instance, primitive) over all
@@ -29,7 +41,7 @@ namespace mb {
 constexpr int WIDE_STACK = 64;
 
 // The traversal stack of one ray. The node group being visited lives in
-// registers (WideTracer::ngBase/ngImask/ngHits, pgBase/pgHits); pushed groups
+// registers (WideTracer::ngBase/ngMask, pgBase/pgHits); pushed groups
 // go to this per-thread array in local memory, which the L1 cache serves.
 // (Keeping the first 4, 8 or 16 entries in shared memory instead, thread-
 // interleaved, measured 5-7 % slower in the trace kernel on the B200.)
@@ -38,35 +50,75 @@ struct LocalStack {
 	MBD void put(int i, uint2 v) { e[i] = v; }
 	MBD uint2 get(int i) const { return e[i]; }
 };
-constexpr uint32_t PRIM_GROUP = 0x80000000u;
-// Primitive masks use bits 0..8*leafMax-1; bit 31 tags primitive groups.
-static_assert(8 * WIDE_LEAF_MAX <= 31 && 8 * WIDE_TLAS_LEAF_MAX <= 31, "primitive mask width");
+// A node group is (child base, hit children in bits 24-31 | internal-slot mask
+// in bits 0-7), a primitive group (primitive base, primitive bits 0-23): what
+// is popped from the stack is a node group exactly when it exceeds PRIM_BITS.
+constexpr uint32_t PRIM_BITS = 0x00FFFFFFu;
+static_assert(8 * WIDE_LEAF_MAX <= 24 && 8 * WIDE_TLAS_LEAF_MAX <= 24, "primitive mask width");
 
-MBD uint32_t octant_flip(f3 d) {
-	return 7u ^ ((d.x < 0.0f ? 4u : 0u) | (d.y < 0.0f ? 2u : 0u) | (d.z < 0.0f ? 1u : 0u));
+// Sign bits of the reciprocal direction (of a zero component's as well).
+MBD uint32_t ray_octant(f3 d) {
+	return (d.x < 0.0f ? 4u : 0u) | (d.y < 0.0f ? 2u : 0u) | (d.z < 0.0f ? 1u : 0u);
+}
+// The root as the only child, in slot 0, of a virtual parent.
+MBD uint32_t root_group(uint32_t oct) { return (1u << (24u + oct)) | 1u; }
+
+// Reciprocal direction for the box tests only, within 1 ulp and clamped as
+// slab_rcp: the box tests need t to a relative 2^-20 (BOX_FAR_SLACK), and an
+// IEEE division is about ten instructions per component.
+MBD float box_rcp(float x) {
+	float r;
+	asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+	return fminf(fmaxf(r, -18446744073709551616.0f), 18446744073709551616.0f);
+}
+MBD f3 box_rcp3(f3 d) { return make3(box_rcp(d.x), box_rcp(d.y), box_rcp(d.z)); }
+
+// Two fused multiply-adds in one instruction (sm_100's packed f32x2 form),
+// each rounded like __fmaf_rn.
+MBD unsigned long long pack2(float a, float b) {
+	unsigned long long v;
+	asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b));
+	return v;
+}
+MBD void fma2(float qa, float qb, unsigned long long s, unsigned long long o, float& ra, float& rb) {
+	unsigned long long v;
+	asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(v) : "l"(pack2(qa, qb)), "l"(s), "l"(o));
+	asm("mov.b64 {%0, %1}, %2;" : "=f"(ra), "=f"(rb) : "l"(v));
 }
 
-// Byte b (0..3) of w as an exact float: 0x4B0000bb is the float 2^23 + bb.
-MBD float qbyte(uint32_t w, int b) {
-	return __fsub_rn(__int_as_float(int(__byte_perm(w, 0x4B000000u, 0x7440u | uint32_t(b)))), 8388608.0f);
+// Byte b (0..3) of w as the float 2^15 + byte: 0x4700bb00. The offset is
+// folded into the additive constant of the box test (below), so a byte costs
+// one instruction.
+constexpr float QBYTE_BIAS = 32768.0f;
+MBD float qbyte_biased(uint32_t w, int b) {
+	return __uint_as_float(__byte_perm(w, 0x47000000u, 0x7404u | (uint32_t(b) << 4)));
 }
 
-// Out-of-line pieces of the traversal loop that run at most a few times per
-// ray (instance transitions) or rarely (non-triangle primitives); keeping them
-// out of the loop body keeps the loop in the instruction cache.
-static __device__ __noinline__ FastRay make_ray_ool(f3 o, f3 d) { return make_ray(o, d); }
-static __device__ __noinline__ InstRay instance_ray_ool(const DScene& S, uint32_t i, f3 o, f3 d) {
-	return instance_ray(load_w2i(S, i), o, d);
-}
+// Primitives other than triangles, out of line (rare in large scenes, and
+// large code). The quad test's exact reciprocal of the dominant direction
+// component is computed here; spheres need none.
 struct PrimHit { float t; f2 uv; bool hit; };
-static __device__ __noinline__ PrimHit other_prim_test(const DLod* l, FastRay r, int p) {
+MBD FastRay other_ray(const DLod& l, f3 o, f3 d, int p) {
+	FastRay r;
+	r.o = o; r.d = d;
+	r.kx = r.ky = r.kz = 0;
+	r.Sx = r.Sy = r.Sz = 0.0f;
+	float inv = 0.0f;
+	if(uint32_t(p) < l.numTriangles + l.numQuads) {
+		const float ax = fabsf(d.x), ay = fabsf(d.y), az = fabsf(d.z);
+		inv = slab_rcp((ax < ay || ax < az) ? (ay >= az ? d.y : d.z) : d.x); // quad_test's axis d0
+	}
+	r.inv = make3(inv, inv, inv);
+	return r;
+}
+static __device__ __noinline__ PrimHit other_prim_test(const DLod* l, f3 o, f3 d, int p) {
 	PrimHit h;
-	h.hit = prim_test(*l, r, 0, p, h.t, h.uv);
+	h.hit = prim_test(*l, other_ray(*l, o, d, p), 0, p, h.t, h.uv);
 	return h;
 }
-static __device__ __noinline__ PrimHit other_prim_test_alpha(const DLod* l, FastRay r, int p, AlphaCtx alpha) {
+static __device__ __noinline__ PrimHit other_prim_test_alpha(const DLod* l, f3 o, f3 d, int p, AlphaCtx alpha) {
 	PrimHit h;
-	h.hit = prim_test(*l, r, 0, p, h.t, h.uv, alpha);
+	h.hit = prim_test(*l, other_ray(*l, o, d, p), 0, p, h.t, h.uv, alpha);
 	return h;
 }
 
@@ -86,24 +138,30 @@ MBD float max3_(float a, float b, float c) {
 // Tests the eight child boxes of node `idx`; returns the child's node group
 // and primitive group. A child is hit when
 //   max(near planes, 0) <= min(far planes * (1 + 2^-20), tmaxBox).
-// The far-plane tolerance is applied to the per-node scale and offset, not per
-// child; that moves a far plane by a few ulp of its t, far less than the grid
-// step of margin every quantised box carries, so the test stays conservative.
-MBD void wide_node_test(const WideNode* nodes, uint32_t idx, const FastRay& r, uint32_t flip, float tmaxBox,
-                        uint32_t& ngBase, uint32_t& ngImask, uint32_t& ngHits, uint32_t& pgBase, uint32_t& pgHits) {
+// With a plane's byte read as q + 2^15, its distance is one multiply-add:
+//   (q + 2^15) * s + (o - 2^15 * s),
+// near and far plane of an axis in one packed instruction. The additive
+// constant is rounded to 2^-9 of a grid step, and the far-plane tolerance is
+// applied to the per-node scale and offset, not per child: both move a plane
+// by far less than the grid step of margin every quantised box carries, so
+// the test stays conservative.
+MBD void wide_node_test(const WideNode* nodes, uint32_t idx, f3 org, f3 inv, uint32_t oct, float tmaxBox,
+                        uint32_t& ngBase, uint32_t& ngMask, uint32_t& pgBase, uint32_t& pgHits) {
 	const float4* q = reinterpret_cast<const float4*>(nodes + idx);
 	const float4 n0 = __ldg(q), n1 = __ldg(q + 1), n2 = __ldg(q + 2), n3 = __ldg(q + 3), n4 = __ldg(q + 4);
 	const uint32_t eim = __float_as_uint(n0.w);
-	const float sx = __fmul_rn(__uint_as_float((eim & 0xFFu) << 23), r.inv.x);
-	const float sy = __fmul_rn(__uint_as_float(((eim >> 8) & 0xFFu) << 23), r.inv.y);
-	const float sz = __fmul_rn(__uint_as_float(((eim >> 16) & 0xFFu) << 23), r.inv.z);
-	const float ox = __fmul_rn(__fsub_rn(n0.x, r.o.x), r.inv.x);
-	const float oy = __fmul_rn(__fsub_rn(n0.y, r.o.y), r.inv.y);
-	const float oz = __fmul_rn(__fsub_rn(n0.z, r.o.z), r.inv.z);
-	const float fsx = __fmul_rn(sx, BOX_FAR_SLACK), fsy = __fmul_rn(sy, BOX_FAR_SLACK), fsz = __fmul_rn(sz, BOX_FAR_SLACK);
-	const float fox = __fmul_rn(ox, BOX_FAR_SLACK), foy = __fmul_rn(oy, BOX_FAR_SLACK), foz = __fmul_rn(oz, BOX_FAR_SLACK);
-	const uint32_t imask = eim >> 24;
-	const bool fx = r.inv.x < 0.0f, fy = r.inv.y < 0.0f, fz = r.inv.z < 0.0f;
+	auto axis = [](float grid, uint32_t ex, float o, float i, unsigned long long& s2, unsigned long long& o2) {
+		const float s = __fmul_rn(__uint_as_float(ex << 23), i);
+		const float t = __fmul_rn(__fsub_rn(grid, o), i);
+		const float fs = __fmul_rn(s, BOX_FAR_SLACK), ft = __fmul_rn(t, BOX_FAR_SLACK);
+		s2 = pack2(s, fs);
+		o2 = pack2(__fmaf_rn(-QBYTE_BIAS, s, t), __fmaf_rn(-QBYTE_BIAS, fs, ft));
+	};
+	unsigned long long sx, sy, sz, ox, oy, oz;
+	axis(n0.x, eim & 0xFFu, org.x, inv.x, sx, ox);
+	axis(n0.y, (eim >> 8) & 0xFFu, org.y, inv.y, sy, oy);
+	axis(n0.z, (eim >> 16) & 0xFFu, org.z, inv.z, sz, oz);
+	const bool fx = (oct & 4u) != 0u, fy = (oct & 2u) != 0u, fz = (oct & 1u) != 0u;
 	const uint32_t lx0 = __float_as_uint(n2.x), lx1 = __float_as_uint(n2.y);
 	const uint32_t ly0 = __float_as_uint(n2.z), ly1 = __float_as_uint(n2.w);
 	const uint32_t lz0 = __float_as_uint(n3.x), lz1 = __float_as_uint(n3.y);
@@ -114,37 +172,36 @@ MBD void wide_node_test(const WideNode* nodes, uint32_t idx, const FastRay& r, u
 	const uint32_t ny[2] = { fy ? hy0 : ly0, fy ? hy1 : ly1 }, fyw[2] = { fy ? ly0 : hy0, fy ? ly1 : hy1 };
 	const uint32_t nz[2] = { fz ? hz0 : lz0, fz ? hz1 : lz1 }, fzw[2] = { fz ? lz0 : hz0, fz ? lz1 : hz1 };
 	const uint32_t meta[2] = { __float_as_uint(n1.z), __float_as_uint(n1.w) };
-	uint32_t nh = 0, ph = 0;
+	uint32_t hits = 0;
 #pragma unroll
-	for(int i = 0; i < 8; ++i) {
-		const int w = i >> 2, b = i & 3;
-		const float tnx = __fmaf_rn(qbyte(nx[w], b), sx, ox);
-		const float tny = __fmaf_rn(qbyte(ny[w], b), sy, oy);
-		const float tnz = __fmaf_rn(qbyte(nz[w], b), sz, oz);
-		const float tfx = __fmaf_rn(qbyte(fxw[w], b), fsx, fox);
-		const float tfy = __fmaf_rn(qbyte(fyw[w], b), fsy, foy);
-		const float tfz = __fmaf_rn(qbyte(fzw[w], b), fsz, foz);
-		const float tnear = max3_(tnx, tny, fmax_(tnz, 0.0f));
-		const float tfar = min3_(tfx, tfy, fmin_(tfz, tmaxBox));
-		if(tnear <= tfar) {
-			if(imask & (1u << i)) {
-				nh |= 1u << (uint32_t(i) ^ flip);
-			} else {
-				const uint32_t m = (meta[w] >> (8 * b)) & 0xFFu;
-				ph |= ((1u << (m >> 5)) - 1u) << (m & 31u);
-			}
+	for(int w = 0; w < 2; ++w) {
+		// four slots at a time: an internal child's bit position (24 + slot,
+		// the only ones with bits 3 and 4 set) is moved into traversal order
+		const uint32_t inner = ((meta[w] & (meta[w] << 1)) & 0x10101010u) >> 4;
+		const uint32_t pos = meta[w] ^ (oct * inner);
+		const uint32_t bits = (meta[w] >> 5) & 0x07070707u;
+#pragma unroll
+		for(int b = 0; b < 4; ++b) {
+			float tnx, tny, tnz, tfx, tfy, tfz;
+			fma2(qbyte_biased(nx[w], b), qbyte_biased(fxw[w], b), sx, ox, tnx, tfx);
+			fma2(qbyte_biased(ny[w], b), qbyte_biased(fyw[w], b), sy, oy, tny, tfy);
+			fma2(qbyte_biased(nz[w], b), qbyte_biased(fzw[w], b), sz, oz, tnz, tfz);
+			const float tnear = max3_(tnx, tny, fmax_(tnz, 0.0f));
+			const float tfar = min3_(tfx, tfy, fmin_(tfz, tmaxBox));
+			// (a funnel shift takes its distance modulo 32: the low five bits of the slot's byte)
+			const uint32_t m = __funnelshift_l(0u, __byte_perm(bits, 0u, 0x4440u | uint32_t(b)), pos >> (8 * b));
+			if(tnear <= tfar) hits |= m;
 		}
 	}
 	ngBase = __float_as_uint(n1.x);
-	ngImask = imask;
-	ngHits = nh;
+	ngMask = (hits & ~PRIM_BITS) | (eim >> 24);
 	pgBase = __float_as_uint(n1.y);
-	pgHits = ph;
+	pgHits = hits & PRIM_BITS;
 }
 
-// Resumable traversal of one ray: init() sets it up, every step() visits at
-// most one node and that node's hit primitives (or enters / leaves an
-// instance), and returns true once the ray is finished. Kernels that refill
+// Resumable traversal of one ray: init() sets it up, every step() enters a
+// pending instance, visits at most one node and that node's hit primitives
+// and leaves a finished instance, and returns true once the ray is finished. Kernels that refill
 // lanes as soon as their ray finishes call step() from one loop shared by the
 // whole warp. Alpha mode AM: ALPHA_NEVER, every surface is opaque (scenes
 // without alpha textures, and the wireframe renderer's
@@ -154,50 +211,71 @@ MBD void wide_node_test(const WideNode* nodes, uint32_t idx, const FastRay& r, u
 enum AlphaMode { ALPHA_NEVER = 0, ALPHA_ALWAYS = 1, ALPHA_SCENE = 2 };
 template < int AM >
 struct WideTracerT {
-	FastRay wr;           // world ray, prepared (wr.o, wr.d: the ray as given)
-	FastRay r;            // ray of the current level
+	f3 wo, wd;            // world ray as given
+	f3 o, d, inv;         // ray of the current level (d: object level only)
+	int kx, ky, kz;       // shear axes and constants of the triangle test (object level)
+	float Sx, Sy, Sz;
 	float scale;          // object-space length of a world-space unit
-	float tmaxW;          // shadow rays: world-space segment length
-	HitRec best;          // closest hit so far (best.t holds the incoming tmax)
-	const DLod* lod;
+	float t;              // closest hit so far, or the incoming tmax; shadow rays: the segment's length
+	f2 sp2;               // its surface parameters
+	int hitInst, hitPrim; // -1: none yet
 	const WideNode* nodes;
-	uint32_t flip, ngBase, ngImask, ngHits, pgBase, pgHits;
+	const float4* soup;
+	uint32_t oct, ngBase, ngMask, pgBase, pgHits;
 	int inst, sp, instSp, steps; // steps: what is left of the scene's step limit
-	bool any, single, occluded, done;
+	bool any, done;
+
+	MBD HitRec hit() const {
+		HitRec h;
+		h.t = t; h.inst = hitInst; h.prim = hitPrim; h.sp = sp2; h.has = hitInst >= 0;
+		return h;
+	}
+	MBD bool occluded() const { return hitInst >= 0; } // of a shadow ray
 
 	template < class C >
-	MBD void init(const DScene& S, f3 o, f3 d, float tmax, bool anyHit, C& cnt) {
-		tmaxW = tmax;
+	MBD void init(const DScene& S, f3 org, f3 dir, float tmax, bool anyHit, C&) {
+		wo = org; wd = dir;
 		any = anyHit;
-		occluded = false;
-		best.t = tmax; best.inst = -1; best.prim = -1; best.sp = make2(0.0f, 0.0f); best.has = false;
-		sp = 0; instSp = -1; steps = S.maxSteps; inst = -1; lod = nullptr;
-		scale = 1.0f;
-		ngBase = 0; ngImask = 1; ngHits = 0; pgBase = 0; pgHits = 0;
-		single = S.activeInstances == 1;
+		t = tmax; hitInst = -1; hitPrim = -1; sp2 = make2(0.0f, 0.0f);
+		sp = 0; instSp = -1; steps = S.maxSteps; inst = -1;
+		ngBase = 0; ngMask = 0; pgBase = 0; pgHits = 0;
 		done = S.activeInstances <= 0;
-		if(done) return;
-		wr = make_ray_ool(o, d);
-		r = wr;
-		flip = octant_flip(d);
-		nodes = S.tlasWide;
-		if(single) enter(S, uint32_t(S.validInstance), cnt);
-		else ngHits = S.tlasNumWide > 0 ? (1u << flip) : 0u;
+		if(S.activeInstances == 1) pgHits = 1u; // its instance is entered by the first step
+		else if(S.tlasNumWide > 0) { to_world(S); ngMask = root_group(oct); }
 	}
 
+	// Sets the world ray and the instance level's hierarchy.
+	MBD void to_world(const DScene& S) {
+		o = wo;
+		inv = box_rcp3(wd);
+		oct = ray_octant(inv);
+		scale = 1.0f;
+		nodes = S.tlasWide;
+		instSp = -1;
+	}
+
+	// Transforms the ray into instance i's object space (the arithmetic of
+	// instance_ray and make_ray) and starts at its hierarchy's root.
 	template < class C >
 	MBD void enter(const DScene& S, uint32_t i, C& cnt) {
 		++cnt.instances;
 		inst = int(i);
-		lod = S.lods + __ldg(S.instanceLod + i);
-		const InstRay ir = instance_ray_ool(S, i, wr.o, wr.d);
-		r = ir.ray;
-		scale = ir.scale;
-		flip = octant_flip(r.d);
-		nodes = lod->wnodes;
-		const int np = lod->numPrims;
-		ngBase = 0; ngImask = 1; ngHits = 0; pgBase = 0; pgHits = 0;
-		if(np >= 2) ngHits = 1u << flip; // the root, slot 0 of a virtual parent
+		const float4* rec = reinterpret_cast<const float4*>(S.instRecs + i);
+		Mat34 W;
+		W.r0 = __ldg(rec); W.r1 = __ldg(rec + 1); W.r2 = __ldg(rec + 2);
+		const ulonglong2 ptr = __ldg(reinterpret_cast<const ulonglong2*>(rec + 3));
+		const int np = __ldg(reinterpret_cast<const int*>(rec + 4));
+		nodes = reinterpret_cast<const WideNode*>(ptr.x);
+		soup = reinterpret_cast<const float4*>(ptr.y);
+		const f3 dirO = xform_dir(W, wd);
+		scale = len(dirO);
+		o = xform_point(W, wo);
+		d = dirO / scale;
+		inv = box_rcp3(d);
+		oct = ray_octant(inv);
+		shear(d, kx, ky, kz, Sx, Sy, Sz);
+		ngBase = 0; ngMask = 0; pgBase = 0; pgHits = 0;
+		if(np >= 2) ngMask = root_group(oct);
 		else if(np == 1) pgHits = 1u;
 		instSp = sp;
 	}
@@ -220,80 +298,79 @@ struct WideTracerT {
 	MBD bool step_impl(const DScene& S, C& cnt, Stack& stack) {
 		if(done) return true;
 		if(--steps < 0) { ++cnt.errors; done = true; return true; }
-		if(ngHits) {
-			const uint32_t k = uint32_t(__ffs(int(ngHits)) - 1);
-			ngHits &= ngHits - 1u;
-			const uint32_t s = k ^ flip;
-			const uint32_t child = ngBase + uint32_t(__popc(ngImask & ((1u << s) - 1u)));
-			if(ngHits) {
+		if(instSp < 0 && pgHits) {
+			// instance leaves of the top level: enter one, keep the rest
+			uint32_t id = S.validInstance;
+			if(S.activeInstances != 1) {
+				const uint32_t j = 31u - uint32_t(__clz(int(pgHits)));
+				id = uint32_t(__ldg(S.tlasWidePrims + pgBase + j));
+				pgHits ^= 1u << j;
+				if(sp + 2 > WIDE_STACK) { ++cnt.errors; done = true; return true; }
+				if(ngMask > PRIM_BITS) stack.put(sp++, make_uint2(ngBase, ngMask));
+				if(pgHits) stack.put(sp++, make_uint2(pgBase, pgHits));
+			}
+			enter(S, id, cnt);
+		}
+		if(ngMask > PRIM_BITS) {
+			const uint32_t k = 31u - uint32_t(__clz(int(ngMask))); // highest bit first: nearest octant first
+			const uint32_t s = (k ^ oct) & 7u;
+			const uint32_t child = ngBase + uint32_t(__popc(ngMask & ((1u << s) - 1u)));
+			ngMask ^= 1u << k;
+			if(ngMask > PRIM_BITS) {
 				if(sp >= WIDE_STACK) { ++cnt.errors; done = true; return true; }
-				stack.put(sp++, make_uint2(ngBase, ngImask | (ngHits << 8)));
+				stack.put(sp++, make_uint2(ngBase, ngMask));
 			}
 			++cnt.nodes;
-			const float tmaxBox = (any ? tmaxW : best.t) * scale * BOX_SLACK;
-			wide_node_test(nodes, child, r, flip, tmaxBox, ngBase, ngImask, ngHits, pgBase, pgHits);
+			const float tmaxBox = t * scale * BOX_SLACK;
+			wide_node_test(nodes, child, o, inv, oct, tmaxBox, ngBase, ngMask, pgBase, pgHits);
 		}
-		if(pgHits) {
-			if(instSp >= 0) {
-				const float4* soup = lod->wsoup;
-				const uint32_t ntri = lod->numTriangles;
-				do {
-					const uint32_t j = uint32_t(__ffs(int(pgHits)) - 1);
-					pgHits &= pgHits - 1u;
-					// all three rows at once (every primitive has them), so a
-					// triangle costs one round trip to memory, not two
-					const float4* s4 = soup + 3 * size_t(pgBase + j);
-					const float4 a = __ldg(s4), b = __ldg(s4 + 1), c = __ldg(s4 + 2);
-					const int p = __float_as_int(a.w);
-					++cnt.prims;
-					float t;
-					f2 uv;
-					bool hit;
-					if(uint32_t(p) < ntri) {
-						hit = tri_test(r, f4to3(a), f4to3(b), f4to3(c), t, uv) && t > 0.0f;
-						if(ALPHA && hit) hit = !alpha_cuts_triangle(alpha_ctx(S), *lod, p, uv);
+		if(instSp >= 0 && pgHits) {
+			do {
+				const uint32_t j = 31u - uint32_t(__clz(int(pgHits)));
+				pgHits ^= 1u << j;
+				// all three rows at once (every primitive has them), so a
+				// triangle costs one round trip to memory, not two
+				const float4* s4 = soup + 3 * size_t(pgBase + j);
+				const float4 a = __ldg(s4), b = __ldg(s4 + 1), c = __ldg(s4 + 2);
+				const int p = __float_as_int(a.w);
+				++cnt.prims;
+				float to;
+				f2 uv;
+				bool hit;
+				if(__float_as_int(b.w) == SOUP_TRIANGLE) {
+					hit = tri_test(o, kx, ky, kz, Sx, Sy, Sz, f4to3(a), f4to3(b), f4to3(c), to, uv) && to > 0.0f;
+					if(ALPHA && hit) hit = !alpha_cuts_triangle(alpha_ctx(S), lod(S), p, uv);
+				} else {
+					const PrimHit ph = ALPHA ? other_prim_test_alpha(&lod(S), o, d, p, alpha_ctx(S)) : other_prim_test(&lod(S), o, d, p);
+					hit = ph.hit; to = ph.t; uv = ph.uv;
+				}
+				if(hit) {
+					if(any) {
+						if(to < t * scale) { hitInst = inst; done = true; return true; }
 					} else {
-						const PrimHit ph = ALPHA ? other_prim_test_alpha(lod, r, p, alpha_ctx(S)) : other_prim_test(lod, r, p);
-						hit = ph.hit; t = ph.t; uv = ph.uv;
-					}
-					if(hit) {
-						if(any) {
-							if(t < tmaxW * scale) { occluded = true; done = true; return true; }
-						} else {
-							const float tw = __fdiv_rn(t, scale);
-							if(better(tw, inst, p, best)) { best.t = tw; best.inst = inst; best.prim = p; best.sp = uv; best.has = true; }
+						const float tw = __fdiv_rn(to, scale);
+						// better(): with no hit yet (hitInst -1) equal distances do not count
+						if(tw < t || (tw == t && (inst < hitInst || (inst == hitInst && p < hitPrim)))) {
+							t = tw; hitInst = inst; hitPrim = p; sp2 = uv;
 						}
 					}
-				} while(pgHits);
-			} else {
-				// instance leaves of the top level: enter one, keep the rest
-				const uint32_t j = uint32_t(__ffs(int(pgHits)) - 1);
-				pgHits &= pgHits - 1u;
-				const uint32_t id = uint32_t(__ldg(S.tlasWidePrims + pgBase + j));
-				if(sp + 2 > WIDE_STACK) { ++cnt.errors; done = true; return true; }
-				if(ngHits) stack.put(sp++, make_uint2(ngBase, ngImask | (ngHits << 8)));
-				if(pgHits) stack.put(sp++, make_uint2(pgBase, pgHits | PRIM_GROUP));
-				enter(S, id, cnt);
-				return false;
-			}
+				}
+			} while(pgHits);
 		}
-		if(!ngHits) {
+		if(ngMask <= PRIM_BITS && !pgHits) {
 			if(instSp >= 0 && sp == instSp) {
-				if(single) { done = true; return true; }
-				r = wr;
-				flip = octant_flip(wr.d);
-				scale = 1.0f;
-				nodes = S.tlasWide;
-				instSp = -1;
+				if(S.activeInstances == 1) { done = true; return true; }
+				to_world(S);
 			}
 			if(sp == 0) { done = true; return true; }
 			const uint2 e = stack.get(--sp);
-			if(e.y & PRIM_GROUP) { pgBase = e.x; pgHits = e.y & ~PRIM_GROUP; }
-			else { ngBase = e.x; ngImask = e.y & 0xFFu; ngHits = e.y >> 8; }
+			if(e.y > PRIM_BITS) { ngBase = e.x; ngMask = e.y; }
+			else { pgBase = e.x; pgHits = e.y; }
 		}
 		return false;
 	}
 
+	MBD const DLod& lod(const DScene& S) const { return S.lods[__ldg(S.instanceLod + inst)]; }
 };
 
 using WideTracer = WideTracerT<ALPHA_SCENE>;
@@ -305,7 +382,7 @@ MBD HitRec closest_hit_wide(const DScene& S, f3 o, f3 dir, float tmax, C& cnt, S
 	WideTracerT<AM> t;
 	t.init(S, o, dir, tmax, false, cnt);
 	while(!t.step(S, cnt, stack)) {}
-	return t.best;
+	return t.hit();
 }
 
 // Occlusion of a prepared shadow ray (origin offset, unit direction, length tmax).
@@ -315,7 +392,7 @@ MBD bool occluded_wide(const DScene& S, f3 a, f3 dir, float tmax, C& cnt, Stack&
 	WideTracerT<ALPHA_SCENE> t;
 	t.init(S, a, dir, tmax, true, cnt);
 	while(!t.step(S, cnt, stack)) {}
-	return t.occluded;
+	return t.occluded();
 }
 
 } // namespace mb
