@@ -98,24 +98,26 @@ __global__ void k_tight_boxes(const DLod* lods, const uint32_t* instLod, const f
 	}
 }
 
-__global__ void k_instance_records(const DLod* lods, const uint32_t* instLod, const float4* w2i, uint32_t n, InstRec* out) {
-	const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-	if(i >= n) return;
+__global__ void k_instance_records(const DLod* lods, const uint32_t* instLod, const float4* w2i, const int32_t* slotInst,
+                                   int32_t single, uint32_t slots, InstRec* out) {
+	const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+	if(k >= slots) return;
+	const size_t i = size_t(slotInst ? slotInst[k] : single);
 	const uint32_t li = instLod[i];
 	InstRec r;
-	r.r0 = w2i[3 * size_t(i)]; r.r1 = w2i[3 * size_t(i) + 1]; r.r2 = w2i[3 * size_t(i) + 2];
-	r.nodes = nullptr; r.soup = nullptr; r.numPrims = 0;
-	r.pad[0] = r.pad[1] = r.pad[2] = 0;
+	r.r0 = w2i[3 * i]; r.r1 = w2i[3 * i + 1]; r.r2 = w2i[3 * i + 2];
+	r.nodes = nullptr; r.soup = nullptr; r.numPrims = 0; r.inst = int32_t(i);
+	r.pad[0] = r.pad[1] = 0;
 	if(li != 0xFFFFFFFFu) { r.nodes = lods[li].wnodes; r.soup = lods[li].wsoup; r.numPrims = lods[li].numPrims; }
-	out[i] = r;
+	out[k] = r;
 }
 
 } // namespace
 
-cudaError_t instance_records(const DLod* lods, const uint32_t* instLod, const float4* w2i, uint32_t n, InstRec* out,
-                             cudaStream_t stream) {
-	if(n == 0) return cudaSuccess;
-	k_instance_records<<<(n + 127) / 128, 128, 0, stream>>>(lods, instLod, w2i, n, out);
+cudaError_t instance_records(const DLod* lods, const uint32_t* instLod, const float4* w2i, const int32_t* slotInst,
+                             int32_t single, uint32_t slots, InstRec* out, cudaStream_t stream) {
+	if(slots == 0) return cudaSuccess;
+	k_instance_records<<<(slots + 127) / 128, 128, 0, stream>>>(lods, instLod, w2i, slotInst, single, slots, out);
 	return cudaGetLastError();
 }
 

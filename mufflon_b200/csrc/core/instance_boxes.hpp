@@ -16,8 +16,9 @@ namespace mb {
 cudaError_t tight_instance_boxes(const DLod* lods, const uint32_t* instLod, const float* instToWorld, uint32_t n,
                                  const float* looseBoxes, float* out, cudaStream_t stream);
 
-// out[i] = what a ray needs to enter instance i (masked instances: no object).
-cudaError_t instance_records(const DLod* lods, const uint32_t* instLod, const float4* w2i, uint32_t n, InstRec* out,
-                             cudaStream_t stream);
+// out[k] = what a ray needs to enter the instance slotInst[k] (slotInst null:
+// the instance `single`) of leaf slot k.
+cudaError_t instance_records(const DLod* lods, const uint32_t* instLod, const float4* w2i, const int32_t* slotInst,
+                             int32_t single, uint32_t slots, InstRec* out, cudaStream_t stream);
 
 } // namespace mb

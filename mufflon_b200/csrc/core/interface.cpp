@@ -1464,11 +1464,21 @@ Boolean render_iterate(MufflonInstanceHdl h, ProcessTime* iterTime, ProcessTime*
 	CHECK_CUDA(cudaStreamSynchronize(I.stream));
 	if(!r.megakernel) {
 		// next iteration's plan: the first bounce >= wavefrontBounces whose
-		// extension queue held at most tailPaths paths (none: no tail)
+		// extension queue held at most tailPaths paths and whose remaining
+		// vertices cost less in the tail launch than in launches of their own
+		// (none: no tail). A plan stays while it is near that line, so that the
+		// captured graph is not made again for a queue that varies about it.
 		const int maxB = std::max(1, r.params.maxPathLength);
+		const bool same = planKey == r.planKey;
 		int plan = maxB;
-		for(int b = std::max(0, r.wavefrontBounces); b + 1 < maxB && b < int(WF_BOUNCE_STATS); ++b)
-			if(bounceQueue[b] <= unsigned(std::max(0, r.tailPaths))) { plan = b; break; }
+		for(int b = std::max(0, r.wavefrontBounces); b + 1 < maxB && b < int(WF_BOUNCE_STATS); ++b) {
+			if(bounceQueue[b] <= unsigned(std::max(0, r.tailPaths)) &&
+			   tail_pays(bounceQueue[b], b > 0 ? bounceQueue[b - 1] : 0u, maxB - 1 - b, std::max(1, r.params.neeCount),
+			             same && r.plannedTail == b ? 1.5f : 1.0f)) {
+				plan = b;
+				break;
+			}
+		}
 		r.plannedTail = plan;
 		r.planKey = planKey;
 	}

@@ -356,11 +356,6 @@ bool build_device_scene(MufflonInstance& inst, std::string& err) {
 	if(!upload(D.dInstBoxes, D.cap[3], boxes.data(), size_t(numInst) * 6, s, err)) return false;
 	if(!upload(D.dInstCentroids, D.cap[4], cents.data(), size_t(numInst) * 3, s, err)) return false;
 	if(!upload(D.dInstI2W, D.lightCap[0], i2wAll.data(), size_t(numInst) * 12, s, err)) return false;
-	if(!reserve_device(D.dInstRecs, D.cap[12], numInst, err)) return false;
-	{
-		const cudaError_t e = instance_records(D.dLods, D.dInstLod, D.dW2I, numInst, D.dInstRecs, s);
-		if(e != cudaSuccess) { err = std::string("instance records failed: ") + cudaGetErrorString(e); return false; }
-	}
 	if(active > 1) {
 		SceneBuildInput sin{};
 		sin.numInstances = numInst; sin.activeInstances = uint32_t(active);
@@ -373,6 +368,12 @@ bool build_device_scene(MufflonInstance& inst, std::string& err) {
 		sin.wideBoxes = D.dWideInstBoxes;
 		e = inst.builder.build_scene(sin, D.tlas, s);
 		if(e != cudaSuccess) { err = std::string("instance BVH build failed: ") + cudaGetErrorString(e); return false; }
+	}
+	if(active > 0) {
+		if(!reserve_device(D.dInstRecs, D.cap[12], size_t(active), err)) return false;
+		const cudaError_t e = instance_records(D.dLods, D.dInstLod, D.dW2I, active > 1 ? D.tlas.wprims : nullptr, int32_t(valid),
+		                                       uint32_t(active), D.dInstRecs, s);
+		if(e != cudaSuccess) { err = std::string("instance records failed: ") + cudaGetErrorString(e); return false; }
 	}
 	st3(D.aabb, sceneBox.mn); st3(D.aabb + 3, sceneBox.mx);
 	const float instMs = msSince(tInst);

@@ -293,7 +293,7 @@ enum { BPTW_EXT0 = 0, BPTW_SH0 = 2, BPTW_WORK = 4 };
 // 12 blocks (42 registers, more spills) fell back to 715 and 497.
 constexpr int BPTW_SHADE_BLOCKS = 8;
 // ... and the trace stage (5 and 6 measured alike; 8 was 6 % slower).
-constexpr int BPTW_TRACE_BLOCKS = 6;
+constexpr int BPTW_TRACE_BLOCKS = 5;
 // Resident blocks per SM of the connection kernels (k_bptw_connect,
 // k_vcmw_connect) and of VCM's merge kernel. Measured at 1080p (Mrays/s,
 // connections at 8 / 6 / 4 blocks): BPT 778 / 780 / 785, VCM 569 / 569 / 571;
@@ -347,15 +347,14 @@ __global__ void __launch_bounds__(128, BPTW_TRACE_BLOCKS) k_bptw_trace(const DSc
 	Q.nExt = *reinterpret_cast<volatile unsigned*>(W.counters + BPTW_EXT0 + q);
 	Q.nSh = *reinterpret_cast<volatile unsigned*>(W.counters + BPTW_SH0 + q);
 	Q.work = W.counters + BPTW_WORK + gen;
-	trace_ray_queue<AM>(S, Q, counters, [&](unsigned s, bool occluded) {
-		const uint4 meta = __ldcs(W.sMeta + s);
-		float4 add;
-		if(occluded) add = bpt_zeros(meta.w);
-		else {
-			add = __ldcs(W.sAdd + s);
-			bpt_add(T, meta.x, add);
-		}
+	trace_ray_queue<AM>(S, Q, counters, [&](unsigned s, unsigned& pix, float4& add) {
+		pix = __ldcs(W.sMeta + s).x;
+		add = __ldcs(W.sAdd + s);
+	}, [&](unsigned s, unsigned pix, float4 add, bool occluded) {
+		if(!occluded) bpt_add(T, pix, add);
 		if(T.recPixel) {
+			const uint4 meta = __ldcs(W.sMeta + s);
+			if(occluded) add = bpt_zeros(meta.w);
 			const size_t slot = size_t(meta.y) | (size_t(meta.z) << 32);
 			T.recPixel[slot] = int(meta.x);
 			float* o = T.recValue + 4 * slot;

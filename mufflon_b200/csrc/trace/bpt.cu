@@ -236,23 +236,23 @@ __global__ void __launch_bounds__(128, 4) k_bpt(const DScene S, const LtParams P
 		++cnt.rays;
 		if(shadow) ++cnt.shadow;
 		WideTracerT<AM> t;
-		t.init(S, ro, rd, tmax, shadow, cnt);
+		t.init(S, ro, rd, tmax, shadow, stack);
 		while(!t.step(S, cnt, stack)) {}
 		if(shadow) {
-			const float4 add = t.occluded() ? bpt_zeros(conn.zeroSigns) : conn.add;
-			if(!t.occluded()) bpt_add(T, conn.pix, add);
+			const float4 add = t.occluded ? bpt_zeros(conn.zeroSigns) : conn.add;
+			if(!t.occluded) bpt_add(T, conn.pix, add);
 			rec.put(size_t(viewLen) * size_t(maxP) + size_t(l), conn.pix, add);
 			++l;
 		} else if(phase == BP_LWALK) {
-			if(!t.hit().has) start_view();
+			if(!t.hit(stack).has) start_view();
 			else {
-				bpt_new_vertex<false>(S, lp[lightLen], ro, rd, t.hit(), segPdf, lthr, lp[lightLen + 1]);
+				bpt_new_vertex<false>(S, lp[lightLen], ro, rd, t.hit(stack), segPdf, lthr, lp[lightLen + 1]);
 				++lightLen;
 				if(lightLen >= maxP - 1) start_view();
 			}
 		} else {
 			const int nxt = 1 - cur;
-			bpt_new_vertex<false>(S, vp[cur], ro, rd, t.hit(), segPdf, thr, vp[nxt]);
+			bpt_new_vertex<false>(S, vp[cur], ro, rd, t.hit(stack), segPdf, thr, vp[nxt]);
 			++viewLen;
 			cur = nxt;
 			const BV& h = vp[cur];

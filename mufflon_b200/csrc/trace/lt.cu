@@ -212,10 +212,10 @@ __global__ void __launch_bounds__(128, 6) k_lt(const DScene S, const LtParams P,
 			++cnt.rays;
 			if(shadow) ++cnt.shadow;
 			WideTracerT<AM> t;
-			t.init(S, ro, rd, tmax, shadow, cnt);
+			t.init(S, ro, rd, tmax, shadow, stack);
 			while(!t.step(S, cnt, stack)) {}
 			if(shadow) {
-				if(!t.occluded()) {
+				if(!t.occluded) {
 					atomicAdd(T.iter + pix, add);
 					if(T.density) atomicAdd(T.iterDensity + pix, dens);
 					if(T.recPixel) {
@@ -225,11 +225,11 @@ __global__ void __launch_bounds__(128, 6) k_lt(const DScene S, const LtParams P,
 						o[0] = add.x; o[1] = add.y; o[2] = add.z; o[3] = add.w; o[4] = dens;
 					}
 				}
-			} else if(!t.hit().has) {
+			} else if(!t.hit(stack).has) {
 				T.rngState[ph.photon] = ph.rng;
 				phase = PH_IDLE;
 			} else {
-				const Intersection hit = hit_attributes(S, ro, rd, t.hit());
+				const Intersection hit = hit_attributes(S, ro, rd, t.hit(stack));
 				ph.position = ro + rd * hit.distance;
 				ph.ts = tangent_space(S, hit);
 				ph.mat = fetch_material(S, material_index(S, hit.inst, hit.prim), hit.uv);
@@ -364,14 +364,16 @@ __global__ void __launch_bounds__(128, LTW_TRACE_BLOCKS) k_ltw_trace(const DScen
 	Q.nExt = *reinterpret_cast<volatile unsigned*>(W.counters + LTW_EXT0 + q);
 	Q.nSh = *reinterpret_cast<volatile unsigned*>(W.counters + LTW_SH0 + q);
 	Q.work = W.counters + LTW_WORK + gen;
-	trace_ray_queue<AM>(S, Q, counters, [&](unsigned s, bool occluded) {
+	trace_ray_queue<AM>(S, Q, counters, [&](unsigned s, unsigned& pix, float4& add) {
+		pix = __ldcs(W.sMeta + s).x;
+		add = __ldcs(W.sAdd + s);
+	}, [&](unsigned s, unsigned pix, float4 add, bool occluded) {
 		if(occluded) return;
-		const float4 add = __ldcs(W.sAdd + s);
-		const uint2 meta = __ldcs(W.sMeta + s);
-		atomicAdd(T.iter + meta.x, add);
-		const float dens = __ldcs(W.sDir + s).w;
-		if(T.density) atomicAdd(T.iterDensity + meta.x, dens);
+		atomicAdd(T.iter + pix, add);
+		if(T.density) atomicAdd(T.iterDensity + pix, __ldcs(W.sDir + s).w);
 		if(T.recPixel) {
+			const uint2 meta = __ldcs(W.sMeta + s);
+			const float dens = __ldcs(W.sDir + s).w;
 			T.recPixel[meta.y] = int(meta.x);
 			float* o = T.recValue + 5 * size_t(meta.y);
 			o[0] = add.x; o[1] = add.y; o[2] = add.z; o[3] = add.w; o[4] = dens;

@@ -51,14 +51,15 @@ struct DLod {
 	int32_t numWide;
 };
 
-// What a ray needs to enter an instance, in one place: the world-to-instance
-// rows and the object's traversal hierarchy (entering read instance, object
-// index and object record one after the other before).
+// What a ray needs to enter an instance, in one place and in the order of the
+// 8-wide instance level's leaf slots: the world-to-instance rows and the
+// object's traversal hierarchy (entering read the slot's instance, its object
+// index and the object record one after the other before).
 struct alignas(16) InstRec {
 	float4 r0, r1, r2;
 	const WideNode* nodes;
 	const float4* soup;
-	int32_t numPrims, pad[3];
+	int32_t numPrims, inst, pad[2];
 };
 static_assert(sizeof(InstRec) == 80, "InstRec layout");
 
@@ -113,7 +114,7 @@ struct DScene {
 	uint32_t numLods;
 	const float4* worldToInstance; // 3 float4 (rows) per instance
 	const uint32_t* instanceLod;
-	const InstRec* instRecs;       // per instance (masked ones unset)
+	const InstRec* instRecs;       // per leaf slot of the 8-wide instance level (one instance: slot 0)
 	uint32_t numInstances;
 	int32_t activeInstances;
 	uint32_t validInstance;

@@ -27,6 +27,7 @@
 
 #include <algorithm>
 #include <cooperative_groups.h>
+#include <type_traits>
 
 namespace mb {
 namespace {
@@ -72,6 +73,11 @@ MBD unsigned warp_reserve(unsigned* counter, unsigned want) {
 // origins and directions, so similar node visits and step counts. Only the
 // order changes; each ray's result is written to its own slot, and a
 // closest hit does not depend on when the ray is traced.
+// Off unless asked for ("Ray sort bits"): since the warps refill lanes as they
+// become idle, binned rays trace no faster than in queue order (1080p icosphere
+// 1.94 ms binned, 1.88 in order; 4 096 instances 720p 10.7 and 11.0 ms), and
+// the keys, scan and scatter cost 0.1 ms an iteration (a batch over four
+// scenes: 31.3 ms with 12 key bits, 29.2 without).
 
 // Octahedral cell (3 bits per coordinate) of a unit direction.
 MBD unsigned octa_cell(f3 d) {
@@ -177,6 +183,7 @@ __global__ void k_bin_scatter(WfState W, int qNext, int neeCount, unsigned capac
 // share the queues (path p belongs to job pathJob[p]).
 struct OneScene {
 	static constexpr bool adjoint = false;
+	static constexpr bool perPath = false; // whether scene() and params() depend on the path
 	DScene S;
 	PtParams P;
 	MBD const DScene& scene(int) const { return S; }
@@ -231,6 +238,7 @@ MBD void adjoint_vertex(const AdjointState& A, const DScene& S, int p, f3 e, boo
 // A plain render whose paths also keep the adjoint's bookkeeping.
 struct OneSceneAdjoint {
 	static constexpr bool adjoint = true;
+	static constexpr bool perPath = false;
 	DScene S;
 	PtParams P;
 	AdjointState A;
@@ -240,6 +248,7 @@ struct OneSceneAdjoint {
 };
 struct JobScenes {
 	static constexpr bool adjoint = false;
+	static constexpr bool perPath = true;
 	const DJob* jobs;
 	const uint16_t* pathJob;
 	MBD const DScene& scene(int p) const { return jobs[pathJob[p]].scene; }
@@ -301,33 +310,67 @@ __global__ void k_camera(const DScene S, const PtParams P, WfState W, uint32_t n
 	camera_path(S, P, W, p, int(p % width), int(p / width));
 }
 
-// Block-wide traversal statistics in shared memory, one set per ray kind.
-struct BlockStats { unsigned long long v[2][6]; };
+// Traversal statistics of a trace or tail launch. Rays and abandoned rays are
+// counted per thread and added once per warp at the end; the counting kernel
+// variants (C = LocalCounters) also add every ray's node visits, primitive
+// tests and instance entries, block-wide in shared memory.
+struct BlockStats { unsigned long long v[2][3]; };
+template < class C > constexpr bool counts_nodes = !std::is_same<C, NoCounters>::value;
 template < class C >
-MBD void stats_add(BlockStats& b, int kind, const C& c) {
-	if(c.nodes) atomicAdd(&b.v[kind][0], (unsigned long long)c.nodes);
-	if(c.prims) atomicAdd(&b.v[kind][1], (unsigned long long)c.prims);
-	if(c.instances) atomicAdd(&b.v[kind][2], (unsigned long long)c.instances);
-	atomicAdd(&b.v[kind][3], 1ull);
-	if(c.errors) atomicAdd(&b.v[kind][5], (unsigned long long)c.errors);
+MBD void stats_clear(BlockStats& b) {
+	if constexpr(counts_nodes<C>) {
+		if(threadIdx.x < 6) (&b.v[0][0])[threadIdx.x] = 0ull;
+		__syncthreads();
+	}
+}
+// The counts of one finished ray; cnt keeps only its errors.
+template < class C >
+MBD void stats_add(BlockStats& b, int kind, C& cnt) {
+	if constexpr(counts_nodes<C>) {
+		if(cnt.nodes) atomicAdd(&b.v[kind][0], (unsigned long long)cnt.nodes);
+		if(cnt.prims) atomicAdd(&b.v[kind][1], (unsigned long long)cnt.prims);
+		if(cnt.instances) atomicAdd(&b.v[kind][2], (unsigned long long)cnt.instances);
+		cnt.nodes = 0; cnt.prims = 0; cnt.instances = 0;
+	}
+}
+// All threads of the block, after their last ray.
+template < class C >
+MBD void stats_write(const BlockStats& b, const C& cnt, unsigned rays, unsigned shadowRays, TraceCounters* counters) {
+	rays = __reduce_add_sync(0xffffffffu, rays);
+	shadowRays = __reduce_add_sync(0xffffffffu, shadowRays);
+	const unsigned errors = __reduce_add_sync(0xffffffffu, cnt.errors);
+	if((threadIdx.x & 31u) == 0) {
+		if(rays) atomicAdd(&counters[0].rays, (unsigned long long)rays);
+		if(shadowRays) {
+			atomicAdd(&counters[1].rays, (unsigned long long)shadowRays);
+			atomicAdd(&counters[1].shadowRays, (unsigned long long)shadowRays);
+		}
+		if(errors) atomicAdd(&counters[0].errors, errors);
+	}
+	if constexpr(counts_nodes<C>) {
+		__syncthreads();
+		if(threadIdx.x < 2) {
+			TraceCounters* out = counters + threadIdx.x;
+			atomicAdd(&out->nodeVisits, b.v[threadIdx.x][0]);
+			atomicAdd(&out->primTests, b.v[threadIdx.x][1]);
+			atomicAdd(&out->instanceVisits, b.v[threadIdx.x][2]);
+		}
+	}
 }
 
 // Persistent traversal of one bounce: the extension rays of queue q (closest
 // hit) and the shadow-ray groups written by the previous shade (any hit; one
 // lane runs a path's neeCount rays in order and adds the unoccluded
 // contributions in that order). Idle lanes fetch work items with one atomic
-// per warp once at least `refillLanes` of them are idle (or none is busy);
-// with 32 a warp takes 32 new rays whenever all of its rays are finished,
-// which measured fastest: the ray set-up then runs with all lanes at once.
-// Every loop iteration runs one traversal step in every busy lane.
+// per warp once at least `refillLanes` of them are idle (or none is busy), and
+// every pass of the loop runs one part of a traversal step (warp_step).
 // Queue entries are read and written with streaming (evict-first) accesses so
 // that they do not displace the hierarchies from L2.
 template < int MINB, class SP, class C, int AM >
 __global__ void __launch_bounds__(128, MINB) k_trace(const SP sp, WfState W, int q, int neeCount, int workIdx,
                                                      TraceCounters* counters, int refillLanes, int bounce) {
 	__shared__ BlockStats stats;
-	if(threadIdx.x < 12) (&stats.v[0][0])[threadIdx.x] = 0ull;
-	__syncthreads();
+	stats_clear<C>(stats);
 	if(*reinterpret_cast<volatile unsigned*>(W.counters + C_TAILED)) return; // the tail launch finished the paths
 	if(blockIdx.x == 0 && threadIdx.x == 0) {
 		W.counters[q ^ 1] = 0u;           // filled by this bounce's shade
@@ -340,12 +383,11 @@ __global__ void __launch_bounds__(128, MINB) k_trace(const SP sp, WfState W, int
 	const unsigned nGroups = *reinterpret_cast<volatile unsigned*>(W.counters + C_SHADOW0 + (q ^ 1)) / unsigned(neeCount);
 	const unsigned total = nExt + nGroups;
 	WideTracerT<AM> t;
-	bool active = false, exhausted = false;
-	unsigned item = 0;
+	bool active = false, exhausted = (threadIdx.x & 31u) >= lanes_per_warp(total);
 	unsigned ent = 0;      // the item's extension-queue slot or shadow-ray group
-	int path = 0, ray = 0; // path of the current item
-	f3 radiance = make3(0.0f, 0.0f, 0.0f);
-	float radW = 0.0f;
+	int path = 0, ray = 0; // the item's path (extension rays: batches only, for its scene) and shadow ray
+	f3 sum = make3(0.0f, 0.0f, 0.0f); // the path's radiance if the shadow ray is unoccluded
+	unsigned shadowRays = 0;
 	const unsigned lane = threadIdx.x & 31u;
 	for(;;) {
 		bool seek = false; // look for the next shadow ray of the current group
@@ -363,48 +405,43 @@ __global__ void __launch_bounds__(128, MINB) k_trace(const SP sp, WfState W, int
 			if(lane == unsigned(__ffs(int(idle)) - 1)) base = atomicAdd(W.counters + C_WORK + workIdx, unsigned(__popc(idle)));
 			base = __shfl_sync(0xffffffffu, base, __ffs(int(idle)) - 1);
 			if(idle & (1u << lane)) {
-				item = base + unsigned(__popc(idle & ((1u << lane) - 1u)));
+				const unsigned item = base + unsigned(__popc(idle & ((1u << lane) - 1u)));
 				if(item >= total) {
 					exhausted = true;
 				} else if(item < nExt) {
 					ent = W.ordered ? __ldcs(W.extOrder + item) : item;
 					const float4 o = __ldcs(W.qOrg[q] + ent), d = __ldcs(W.qDir[q] + ent);
-					path = W.qPath[q][ent];
-					cnt = C();
-					t.init(sp.scene(path), f4to3(o), f4to3(d), MAX_SCENE_SIZE, false, cnt);
+					if constexpr(SP::perPath) path = W.qPath[q][ent];
+					t.init(sp.scene(path), f4to3(o), f4to3(d), MAX_SCENE_SIZE, false, stack);
 					active = true;
 				} else {
 					ent = W.ordered ? __ldcs(W.shOrder + (item - nExt)) : item - nExt;
 					path = __ldcs(W.sPath + ent * unsigned(neeCount));
-					const float4 acc = W.rad[path];
-					radiance = f4to3(acc);
-					radW = acc.w;
 					ray = 0;
 					seek = true;
 				}
 			}
 		}
 		if(__all_sync(0xffffffffu, exhausted)) break;
-		if(active && t.step(sp.scene(path), cnt, stack)) {
-			if(item < nExt) {
+		if(t.warp_step(sp.scene(path), cnt, stack, active)) {
+			if(!t.any) {
 				stats_add(stats, 0, cnt);
-				const HitRec h = t.hit();
+				const HitRec h = t.hit(stack);
 				__stcs(W.qHit[q] + ent, make_float4(h.t, __int_as_float(h.has ? h.inst : -1), __int_as_float(h.has ? h.prim : -1), h.sp.x));
 				__stcs(W.qHitSpy[q] + ent, h.sp.y);
 				active = false;
 			} else {
 				stats_add(stats, 1, cnt);
 				const unsigned slot = ent * unsigned(neeCount) + unsigned(ray);
-				if(!t.occluded()) {
-					const float4 c4 = __ldcs(W.sContrib + slot);
-					const f3 c = f4to3(c4);
-					radiance = contribute(radiance, c);
+				if(!t.occluded) {
+					W.rad[path] = pack(sum, 0.0f);
 					if(W.auxIter) {
 						float* a = W.auxIter + size_t(AUX_LIGHT) * W.auxStride + size_t(path);
 						*a = *a + nan_to_zero(__ldcs(W.sDir + slot).w);
 					}
 					if constexpr(SP::adjoint) {
-						const f3 cc = contribute(make3(0.0f, 0.0f, 0.0f), c);
+						const float4 c4 = __ldcs(W.sContrib + slot);
+						const f3 cc = contribute(make3(0.0f, 0.0f, 0.0f), f4to3(c4));
 						adjoint_add(sp.A, path, cc);
 						adjoint_emitted(sp.A, sp.scene(path), path, cc, __float_as_int(c4.w));
 					}
@@ -414,34 +451,26 @@ __global__ void __launch_bounds__(128, MINB) k_trace(const SP sp, WfState W, int
 			}
 		}
 		if(seek) {
-			// next non-empty slot of the group, or write the group's radiance
+			// next non-empty slot of the group
 			active = false;
 			const unsigned g0 = ent * unsigned(neeCount);
 			for(; ray < neeCount; ++ray) {
 				const float4 o = __ldcs(W.sOrg + g0 + unsigned(ray));
 				if(!(o.w > 0.0f)) continue;
 				const float4 d = __ldcs(W.sDir + g0 + unsigned(ray));
-				cnt = C();
-				t.init(sp.scene(path), f4to3(o), f4to3(d), o.w, true, cnt);
+				// The ray's term is added before it is traced, and stored when it
+				// turns out unoccluded: the end of a ray, which most passes of the
+				// loop see in some lane of the warp, then waits for no load. (Only
+				// this lane touches the path's radiance now, in its rays' order.)
+				sum = contribute(f4to3(W.rad[path]), f4to3(__ldcs(W.sContrib + g0 + unsigned(ray))));
+				++shadowRays;
+				t.init(sp.scene(path), f4to3(o), f4to3(d), o.w, true, stack);
 				active = true;
 				break;
 			}
-			if(!active) W.rad[path] = pack(radiance, radW);
 		}
 	}
-	__syncthreads();
-	if(threadIdx.x < 2) {
-		TraceCounters* out = counters + threadIdx.x;
-		const unsigned long long* v = stats.v[threadIdx.x];
-		if(v[3]) {
-			atomicAdd(&out->rays, v[3]);
-			if(threadIdx.x == 1) atomicAdd(&out->shadowRays, v[3]);
-			atomicAdd(&out->nodeVisits, v[0]);
-			atomicAdd(&out->primTests, v[1]);
-			atomicAdd(&out->instanceVisits, v[2]);
-		}
-		if(v[5]) atomicAdd(&out->errors, unsigned(v[5]));
-	}
+	stats_write(stats, cnt, blockIdx.x == 0 && threadIdx.x == 0 ? nExt : 0u, shadowRays, counters);
 }
 
 // One vertex of pt_sample (pt_common.hpp:75-156, random_walk.hpp:38-113):
@@ -689,6 +718,16 @@ MBD void shade_slot(const SP& sp, WfState& W, int q, int bounce, unsigned slot) 
 	if(W.sortBits) bin_append(W.extKey, W.binHist, nslot, ray_key(W, S, sp.group(p), nextO, nextD));
 }
 
+// Whether the tail launch takes the `count` paths of `bounce`, decided alike
+// by the tail and the shade launch of an unplanned iteration; tailBounces: the
+// bounces that may follow, negative where the tail may not take over.
+MBD bool tail_takes(const WfState& W, unsigned count, int bounce, int neeCount, unsigned tailMax, int tailBounces) {
+	if(tailBounces < 0 || count > tailMax) return false;
+	// the trace launches record every bounce's queue length
+	const bool known = bounce > 0 && bounce <= int(WF_BOUNCE_STATS);
+	return tail_pays(count, known ? W.counters[WF_COUNTERS - WF_BOUNCE_STATS + bounce - 1] : 0u, tailBounces, neeCount);
+}
+
 // Shade stage of the wavefront over queue q, grid-stride over its entries
 // (a fixed grid, so that a launch over a short or empty queue costs little).
 // Register budget: 8 resident blocks of 128 threads; the shade is bound by
@@ -696,10 +735,11 @@ MBD void shade_slot(const SP& sp, WfState& W, int q, int bounce, unsigned slot) 
 // made the stage 14 % faster than the unbounded 126-register build (0.44 vs
 // 0.52 ms per 1080p iteration).
 template < class SP >
-__global__ void __launch_bounds__(128, 8) k_shade(const SP sp, WfState W, int q, int bounce, unsigned tailMax, int tailAllowed) {
+__global__ void __launch_bounds__(128, 8) k_shade(const SP sp, WfState W, int q, int bounce, int neeCount,
+                                               unsigned tailMax, int tailBounces) {
 	const unsigned count = *reinterpret_cast<volatile unsigned*>(W.counters + q);
 	if(*reinterpret_cast<volatile unsigned*>(W.counters + C_TAILED)) return;
-	if(tailAllowed && count <= tailMax) {
+	if(tail_takes(W, count, bounce, neeCount, tailMax, tailBounces)) {
 		// the tail launch of this bounce took the paths; later launches skip
 		if(blockIdx.x == 0 && threadIdx.x == 0) W.counters[C_TAILED] = 1u;
 		return;
@@ -719,20 +759,25 @@ __global__ void __launch_bounds__(128, 8) k_shade(const SP sp, WfState W, int q,
 // ends (the warp claims all idle lanes' paths with one atomic), and every pass
 // of the loop traces at most one ray per lane (a shadow ray or the next
 // extension ray) in one traversal loop shared by the warp. A path's random
-// numbers, terms and their order are those of shade_vertex.
+// numbers, terms and their order are those of shade_vertex. It is bound by
+// instruction fetch (ncu: 9.4 of 15 cycles between issues). Running in each
+// pass the one state that most lanes wait in, as warp_step does, raised the
+// lanes per instruction from 2.7 to 5.8 but the time from 0.42 to 0.48 ms
+// (256 x 256 box): the shading code is fetched as often, for fewer paths.
 template < int MINB, class SP, class C, int AM >
 __global__ void __launch_bounds__(128, MINB) k_tail(const SP sp, WfState W, int q, int bounce,
-                                                    int workIdx, TraceCounters* counters, unsigned tailMax) {
+                                                    int workIdx, TraceCounters* counters, int neeCount, unsigned tailMax,
+                                                    int tailBounces) {
 	__shared__ BlockStats stats;
-	if(threadIdx.x < 12) (&stats.v[0][0])[threadIdx.x] = 0ull;
-	__syncthreads();
+	stats_clear<C>(stats);
 	const unsigned count = *reinterpret_cast<volatile unsigned*>(W.counters + q);
-	// takes over only the first bounce whose queue holds at most tailMax paths
-	if(*reinterpret_cast<volatile unsigned*>(W.counters + C_TAILED) || count > tailMax) return;
+	// unplanned (tailBounces >= 0): takes over only the first bounce it pays for
+	if(*reinterpret_cast<volatile unsigned*>(W.counters + C_TAILED)) return;
+	if(tailBounces >= 0 && !tail_takes(W, count, bounce, neeCount, tailMax, tailBounces)) return;
 	enum { T_IDLE = 0, T_NEE, T_WALK, T_EXIT };
 	LocalStack stack;
 	const unsigned lane = threadIdx.x & 31u;
-	int phase = T_IDLE;
+	int phase = lane < lanes_per_warp(count) ? T_IDLE : T_EXIT;
 	int p = 0, b = 0, i = 0;
 	int emitMat = -1; // emitter material of the current shadow ray (adjoint)
 	float guideA = 0.0f, gw = 0.0f, lightTerm = 0.0f; // auxiliary targets: footprint, guide weight, shadow ray's term
@@ -740,6 +785,8 @@ __global__ void __launch_bounds__(128, MINB) k_tail(const SP sp, WfState W, int 
 	float pdfF = 0.0f, radW = 0.0f;
 	u64 rng = 0, neeSeed = 0;
 	ShadeState v;
+	C cnt;
+	unsigned rays = 0, shadowRays = 0;
 	auto on_vertex = [&](f3 e, const VertexInfo& vi) {
 		if constexpr(SP::adjoint) adjoint_vertex(sp.A, sp.scene(p), p, e, vi.surface, vi.materialType, vi.materialIndex, vi.uv, vi.albedo);
 		if(W.auxIter) {
@@ -813,15 +860,16 @@ __global__ void __launch_bounds__(128, MINB) k_tail(const SP sp, WfState W, int 
 				phase = T_IDLE;
 			}
 		}
-		if(!trace) continue;
 		const DScene& S = sp.scene(p);
-		C cnt;
+		if(shadow) ++shadowRays; else if(trace) ++rays;
 		WideTracerT<AM> t;
-		t.init(S, ro, rd, tmax, shadow, cnt);
-		while(!t.step(S, cnt, stack)) {}
+		t.init(S, ro, rd, tmax, shadow, stack);
+		t.done = t.done || !trace;
+		do t.warp_step(S, cnt, stack, true); while(__any_sync(0xffffffffu, !t.done));
+		if(!trace) continue;
 		stats_add(stats, shadow ? 1 : 0, cnt);
 		if(shadow) {
-			if(!t.occluded()) {
+			if(!t.occluded) {
 				radiance = contribute(radiance, c);
 				if constexpr(SP::adjoint) {
 					const f3 cc = contribute(make3(0.0f, 0.0f, 0.0f), c);
@@ -836,22 +884,10 @@ __global__ void __launch_bounds__(128, MINB) k_tail(const SP sp, WfState W, int 
 			++i;
 		} else {
 			++b;
-			begin_vertex(ro, rd, t.hit(), v.position);
+			begin_vertex(ro, rd, t.hit(stack), v.position);
 		}
 	}
-	__syncthreads();
-	if(threadIdx.x < 2) {
-		TraceCounters* out = counters + threadIdx.x;
-		const unsigned long long* v2 = stats.v[threadIdx.x];
-		if(v2[3]) {
-			atomicAdd(&out->rays, v2[3]);
-			if(threadIdx.x == 1) atomicAdd(&out->shadowRays, v2[3]);
-			atomicAdd(&out->nodeVisits, v2[0]);
-			atomicAdd(&out->primTests, v2[1]);
-			atomicAdd(&out->instanceVisits, v2[2]);
-		}
-		if(v2[5]) atomicAdd(&out->errors, unsigned(v2[5]));
-	}
+	stats_write(stats, cnt, rays, shadowRays, counters);
 }
 
 __global__ void k_finalize(WfState W, RenderState R, uint32_t numPixels) {
@@ -1137,7 +1173,7 @@ template < class SP > TraceKernel<SP> trace_kernel(int perSm, bool counting, boo
 }
 
 template < class SP > struct TailKernel {
-	using Fn = void (*)(const SP, WfState, int, int, int, TraceCounters*, unsigned);
+	using Fn = void (*)(const SP, WfState, int, int, int, TraceCounters*, int, unsigned, int);
 	Fn fn;
 	int blocks;
 };
@@ -1215,30 +1251,32 @@ void run_bounces(const SP& sp, WfState W, TraceCounters* counters, uint32_t numP
 			if(b == tuning.tailBounce && b + 1 < maxBounces) {
 				const TailKernel<SP> tl = tail_kernel<SP>(tuning.counters, tuning.alpha);
 				log.begin(WF_TAIL);
-				tl.fn<<<tl.blocks, WF_BLOCK, 0, stream>>>(sp, W, q, b, int(work++), counters, 0xFFFFFFFFu);
+				tl.fn<<<tl.blocks, WF_BLOCK, 0, stream>>>(sp, W, q, b, int(work++), counters, neeCount, 0u, -1);
 				log.end();
 				break;
 			}
 			log.begin(WF_SHADE);
-			k_shade<SP><<<(numPaths + 127) / 128, 128, 0, stream>>>(sp, W, q, b, 0u, 0); // one thread per entry
+			// one thread per entry while the queue is long; a grid for every pixel
+			// takes about 40 us at 1080p however short the queue
+			k_shade<SP><<<b < 2 ? (numPaths + 127) / 128 : shadeGrid, 128, 0, stream>>>(sp, W, q, b, neeCount, 0u, -1);
 			log.end();
 			bin(b);
 			continue;
 		}
 		// From bounce wavefrontBounces on, the first bounce whose queue holds
-		// at most tailMax paths is finished by one launch (decided on the
+		// at most tailMax paths, and pays, is finished by one launch (decided on the
 		// device from the queue length); the later launches return at once.
-		const bool tailAllowed = b >= tuning.wavefrontBounces && b + 1 < maxBounces;
-		if(tailAllowed) {
+		const int tailBounces = b >= tuning.wavefrontBounces && b + 1 < maxBounces ? maxBounces - 1 - b : -1;
+		if(tailBounces >= 0) {
 			const TailKernel<SP> tl = tail_kernel<SP>(tuning.counters, tuning.alpha);
 			log.begin(WF_TAIL);
-			tl.fn<<<tl.blocks, WF_BLOCK, 0, stream>>>(sp, W, q, b, int(work++), counters, tailMax);
+			tl.fn<<<tl.blocks, WF_BLOCK, 0, stream>>>(sp, W, q, b, int(work++), counters, neeCount, tailMax, tailBounces);
 			log.end();
 		}
 		// the shade of this bounce appends to the other queue and to the shadow
 		// queue (the trace launch above reset both counters)
 		log.begin(WF_SHADE);
-		k_shade<SP><<<shadeGrid, 128, 0, stream>>>(sp, W, q, b, tailMax, tailAllowed ? 1 : 0);
+		k_shade<SP><<<shadeGrid, 128, 0, stream>>>(sp, W, q, b, neeCount, tailMax, tailBounces);
 		log.end();
 		bin(b);
 	}

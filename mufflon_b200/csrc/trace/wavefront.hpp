@@ -52,6 +52,31 @@ constexpr int WF_SORT_MAX_BITS = 16;
 constexpr unsigned WF_COUNTERS = 4096;
 constexpr unsigned WF_BOUNCE_STATS = 64;
 
+// Whether the tail launch should finish a queue of `paths` paths, left of the
+// previous bounce's `before` (0: unknown), with up to `bounces` bounces to
+// come. The tail runs a path's vertices one after the other with few lanes
+// per instruction, and worse the longer its paths are; launches of their own
+// cost more per bounce than per vertex. The line was fitted to these times of
+// what remains after two bounces, tail against launches (ms per iteration;
+// paths, share of them that goes on): icosphere 1080p 80 K, 0.09: 0.48 against
+// 0.55 for the next bounce's launches and the tail after it; 64 x 64 box 1.3 K,
+// 0.43: 0.14 and 0.25; plane 1024 x 1024 8 K, 0.02: 0.09 and 0.16; 256 x 256 box
+// 20 K, 0.43: 0.42 and 0.29; cut-outs 613 x 457, two samples, 66 K, 0.39: 1.77
+// and 0.75; 4 096 instances 720p 100 K, 0.5 (after four): the same.
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline bool tail_pays(unsigned paths, unsigned before, int bounces, int neeCount, float slack = 1.0f) {
+	constexpr float TAIL_NS = 5.0f, TAIL_LONG_NS = 8.0f; // per vertex, and more per further vertex of a path
+	constexpr float WAVE_NS = 4.2f, BOUNCE_NS = 32000.0f;
+	const float keep = before > paths ? float(paths) / float(before) : 1.0f;
+	float q = float(paths), vertices = 0.0f, launches = 0.0f;
+	for(int b = 0; b < bounces && q >= 1.0f; ++b) { vertices += q; q *= keep; launches += 1.0f; }
+	const float rays = vertices * 0.5f * float(1 + neeCount);
+	const float further = paths ? vertices / float(paths) - 1.0f : 0.0f;
+	return rays * (TAIL_NS + TAIL_LONG_NS * further) <= slack * (rays * WAVE_NS + launches * BOUNCE_NS);
+}
+
 // WF_EXTEND: the trace launches of the wavefront bounces (extension and
 // shadow rays); WF_TAIL: the launch that finishes the remaining paths.
 // WF_BIN: the scan and scatter launches that order queued rays by coherence.
@@ -75,11 +100,12 @@ struct WfTuning {
 	int traceBlocksPerSm = 6;  // register budget of the trace kernel: 4, 5, 6 or 8 resident blocks of 128 threads
 	int wavefrontBounces = 2;  // bounces 0 .. this-1 always run as separate trace and shade launches; from
 	                           // bounce this on, the first bounce with at most tailPaths queued paths
-	                           // is finished by one launch that runs every remaining path in place
+	                           // that tail_pays() is finished by one launch that runs every remaining
+	                           // path in place
 	int tailPaths = 98304;
 	int tailBounce = -1;       // >= 0: planned schedule, the tail launch takes over at this bounce and
 	                           // nothing is launched after it; -1: decided on the device per bounce
-	int refillLanes = 32;      // idle lanes of a trace warp are refilled together once this many are idle (1..32)
+	int refillLanes = 12;      // idle lanes of a trace warp are refilled together once this many are idle (1..32)
 	int sortBits = 0;          // coherence binning of the queued rays before each trace launch of bounce >= 1
 	int sortDirBits = 3;       // (key bits in all, of them direction bits); 0 bits: trace in queue order
 	int sortGroupBits = 0;     // extra key bits above those for the path's group (batches: the job's scene)

@@ -17,8 +17,8 @@
 // the same arithmetic in every lane) and then that node's hit primitives.
 //
 // What bounds it: divergence and instruction issue (ncu, incoherent bounce of
-// the 1080p icosphere: 7.5 of 32 lanes per instruction, 575 warp instructions
-// per ray, memory below 10 % of its peak), so the step is written for few
+// the icosphere: 50 % of issue slots, 36 % of the ALU pipe, memory below 10 %
+// of its peak; see warp_step), so the step is written for few
 // instructions and registers: box planes from biased bytes in packed
 // multiply-adds, hit masks by shifts of precomputed bytes, approximate
 // reciprocals for boxes, one record per instance, no world-ray shear
@@ -26,7 +26,7 @@
 // an IEEE-reciprocal form with a subtraction per plane byte, out-of-line
 // instance transforms and the prepared world ray in registers (same box, per
 // iteration): trace stage of the 1080p icosphere 2.90 -> 2.12 ms, of 4 096
-// instances at 720p 15.4 -> 14.3 ms; spilled bytes at 80 registers 360 -> 204.
+// instances at 720p 15.4 -> 14.3 ms.
 //
 // The box test cannot cull a box that contains a hit point (wide.hpp), so the
 // closest hit is the minimum of (world t, instance, primitive) over all
@@ -45,8 +45,12 @@ constexpr int WIDE_STACK = 64;
 // go to this per-thread array in local memory, which the L1 cache serves.
 // (Keeping the first 4, 8 or 16 entries in shared memory instead, thread-
 // interleaved, measured 5-7 % slower in the trace kernel on the B200.)
+// The closest hit so far lies beside the stack: it is written when a nearer
+// one is found and read at the end of the ray (or at equal distances).
 struct LocalStack {
 	uint2 e[WIDE_STACK];
+	int2 hit;     // instance (-1: none yet), primitive
+	float2 hitSp; // surface parameters
 	MBD void put(int i, uint2 v) { e[i] = v; }
 	MBD uint2 get(int i) const { return e[i]; }
 };
@@ -199,6 +203,24 @@ MBD void wide_node_test(const WideNode* nodes, uint32_t idx, f3 org, f3 inv, uin
 	pgHits = hits & PRIM_BITS;
 }
 
+// Idle lanes of a persistent warp are refilled together once this many are idle
+// (or none is busy): waiting for all 32 leaves lanes idle behind the longest
+// ray, refilling one by one waits for the queue's loads in most passes. Trace
+// per iteration, icosphere at 1080p and 4 096 instances at 720p: 8 lanes 2.01
+// and 10.1 ms, 12 lanes 1.95 and 10.3 ms, 24 lanes 1.95 and 11.0 ms, all 32
+// 2.11 and 12.4 ms.
+constexpr int REFILL_LANES = 12;
+
+// Lanes of every warp of a persistent launch that take work when `items` do
+// not fill the launch: fewer rays or paths per warp, over more warps, diverge
+// less, and a short queue is bound by the latency of its slowest warp. (64 x
+// 64 box: 0.40 -> 0.27 ms an iteration; the light tracer's short late
+// generations at 1080p: 3.13 -> 2.86 ms.)
+MBD unsigned lanes_per_warp(unsigned items) {
+	const unsigned warps = gridDim.x * (blockDim.x / 32u);
+	return items >= 32u * warps ? 32u : (items + warps - 1u) / warps;
+}
+
 // Resumable traversal of one ray: init() sets it up, every step() enters a
 // pending instance, visits at most one node and that node's hit primitives
 // and leaves a finished instance, and returns true once the ray is finished. Kernels that refill
@@ -213,35 +235,36 @@ template < int AM >
 struct WideTracerT {
 	f3 wo, wd;            // world ray as given
 	f3 o, d, inv;         // ray of the current level (d: object level only)
-	int kx, ky, kz;       // shear axes and constants of the triangle test (object level)
+	uint32_t axes;        // shear axes kx | ky << 2 | kz << 4 and constants of the triangle test (object level)
 	float Sx, Sy, Sz;
 	float scale;          // object-space length of a world-space unit
 	float t;              // closest hit so far, or the incoming tmax; shadow rays: the segment's length
-	f2 sp2;               // its surface parameters
-	int hitInst, hitPrim; // -1: none yet
 	const WideNode* nodes;
 	const float4* soup;
 	uint32_t oct, ngBase, ngMask, pgBase, pgHits;
 	int inst, sp, instSp, steps; // steps: what is left of the scene's step limit
-	bool any, done;
+	bool any, done, occluded;
 
-	MBD HitRec hit() const {
+	template < class Stack >
+	MBD HitRec hit(const Stack& stack) const {
 		HitRec h;
-		h.t = t; h.inst = hitInst; h.prim = hitPrim; h.sp = sp2; h.has = hitInst >= 0;
+		h.t = t; h.inst = stack.hit.x; h.prim = stack.hit.y; h.has = h.inst >= 0;
+		h.sp = h.has ? make2(stack.hitSp.x, stack.hitSp.y) : make2(0.0f, 0.0f);
 		return h;
 	}
-	MBD bool occluded() const { return hitInst >= 0; } // of a shadow ray
 
-	template < class C >
-	MBD void init(const DScene& S, f3 org, f3 dir, float tmax, bool anyHit, C&) {
+	template < class Stack >
+	MBD void init(const DScene& S, f3 org, f3 dir, float tmax, bool anyHit, Stack& stack) {
 		wo = org; wd = dir;
 		any = anyHit;
-		t = tmax; hitInst = -1; hitPrim = -1; sp2 = make2(0.0f, 0.0f);
+		t = tmax; occluded = false;
+		stack.hit = make_int2(-1, -1);
 		sp = 0; instSp = -1; steps = S.maxSteps; inst = -1;
 		ngBase = 0; ngMask = 0; pgBase = 0; pgHits = 0;
 		done = S.activeInstances <= 0;
 		if(S.activeInstances == 1) pgHits = 1u; // its instance is entered by the first step
 		else if(S.tlasNumWide > 0) { to_world(S); ngMask = root_group(oct); }
+		else done = true;
 	}
 
 	// Sets the world ray and the instance level's hierarchy.
@@ -254,17 +277,18 @@ struct WideTracerT {
 		instSp = -1;
 	}
 
-	// Transforms the ray into instance i's object space (the arithmetic of
-	// instance_ray and make_ray) and starts at its hierarchy's root.
+	// Transforms the ray into the object space of the instance in leaf slot
+	// `slot` of the instance level (the arithmetic of instance_ray and
+	// make_ray) and starts at its hierarchy's root.
 	template < class C >
-	MBD void enter(const DScene& S, uint32_t i, C& cnt) {
+	MBD void enter(const DScene& S, uint32_t slot, C& cnt) {
 		++cnt.instances;
-		inst = int(i);
-		const float4* rec = reinterpret_cast<const float4*>(S.instRecs + i);
+		const float4* rec = reinterpret_cast<const float4*>(S.instRecs + slot);
 		Mat34 W;
 		W.r0 = __ldg(rec); W.r1 = __ldg(rec + 1); W.r2 = __ldg(rec + 2);
 		const ulonglong2 ptr = __ldg(reinterpret_cast<const ulonglong2*>(rec + 3));
-		const int np = __ldg(reinterpret_cast<const int*>(rec + 4));
+		const int2 np = __ldg(reinterpret_cast<const int2*>(rec + 4));
+		inst = np.y;
 		nodes = reinterpret_cast<const WideNode*>(ptr.x);
 		soup = reinterpret_cast<const float4*>(ptr.y);
 		const f3 dirO = xform_dir(W, wd);
@@ -273,10 +297,12 @@ struct WideTracerT {
 		d = dirO / scale;
 		inv = box_rcp3(d);
 		oct = ray_octant(inv);
+		int kx, ky, kz;
 		shear(d, kx, ky, kz, Sx, Sy, Sz);
+		axes = uint32_t(kx) | uint32_t(ky) << 2 | uint32_t(kz) << 4;
 		ngBase = 0; ngMask = 0; pgBase = 0; pgHits = 0;
-		if(np >= 2) ngMask = root_group(oct);
-		else if(np == 1) pgHits = 1u;
+		if(np.x >= 2) ngMask = root_group(oct);
+		else if(np.x == 1) pgHits = 1u;
 		instSp = sp;
 	}
 
@@ -294,80 +320,133 @@ struct WideTracerT {
 		}
 	}
 
+	// The parts of a step, for a ray that has something to do there.
+	template < class Stack, class C >
+	MBD void enter_pending(const DScene& S, C& cnt, Stack& stack) {
+		// instance leaves of the top level: enter one, keep the rest
+		const uint32_t j = 31u - uint32_t(__clz(int(pgHits)));
+		const uint32_t slot = pgBase + j;
+		pgHits ^= 1u << j;
+		if(sp + 2 > WIDE_STACK) { ++cnt.errors; done = true; return; }
+		if(ngMask > PRIM_BITS) stack.put(sp++, make_uint2(ngBase, ngMask));
+		if(pgHits) stack.put(sp++, make_uint2(pgBase, pgHits));
+		enter(S, slot, cnt);
+	}
+	template < class Stack, class C >
+	MBD void visit_node(C& cnt, Stack& stack) {
+		const uint32_t k = 31u - uint32_t(__clz(int(ngMask))); // highest bit first: nearest octant first
+		const uint32_t s = (k ^ oct) & 7u;
+		const uint32_t child = ngBase + uint32_t(__popc(ngMask & ((1u << s) - 1u)));
+		ngMask ^= 1u << k;
+		if(ngMask > PRIM_BITS) {
+			if(sp >= WIDE_STACK) { ++cnt.errors; done = true; return; }
+			stack.put(sp++, make_uint2(ngBase, ngMask));
+		}
+		++cnt.nodes;
+		const float tmaxBox = t * scale * BOX_SLACK;
+		wide_node_test(nodes, child, o, inv, oct, tmaxBox, ngBase, ngMask, pgBase, pgHits);
+	}
+	template < bool ALPHA, class Stack, class C >
+	MBD void test_prim(const DScene& S, C& cnt, Stack& stack) {
+		const uint32_t j = 31u - uint32_t(__clz(int(pgHits)));
+		pgHits ^= 1u << j;
+		// all three rows at once (every primitive has them), so a
+		// triangle costs one round trip to memory, not two
+		const float4* s4 = soup + 3 * size_t(pgBase + j);
+		const float4 a = __ldg(s4), b = __ldg(s4 + 1), c = __ldg(s4 + 2);
+		const int p = __float_as_int(a.w);
+		++cnt.prims;
+		float to;
+		f2 uv;
+		bool hit;
+		if(__float_as_int(b.w) == SOUP_TRIANGLE) {
+			hit = tri_test(o, int(axes & 3u), int(axes >> 2 & 3u), int(axes >> 4), Sx, Sy, Sz, f4to3(a), f4to3(b), f4to3(c), to, uv) && to > 0.0f;
+			if(ALPHA && hit) hit = !alpha_cuts_triangle(alpha_ctx(S), lod(S), p, uv);
+		} else {
+			const PrimHit ph = ALPHA ? other_prim_test_alpha(&lod(S), o, d, p, alpha_ctx(S)) : other_prim_test(&lod(S), o, d, p);
+			hit = ph.hit; to = ph.t; uv = ph.uv;
+		}
+		if(hit) {
+			if(any) {
+				if(to < t * scale) { occluded = true; done = true; }
+			} else {
+				const float tw = __fdiv_rn(to, scale);
+				// better(): with no hit yet (instance -1) equal distances do not count
+				if(tw < t || (tw == t && (inst < stack.hit.x || (inst == stack.hit.x && p < stack.hit.y)))) {
+					t = tw; stack.hit = make_int2(inst, p); stack.hitSp = make_float2(uv.x, uv.y);
+				}
+			}
+		}
+	}
+	template < class Stack >
+	MBD void pop(const DScene& S, Stack& stack) {
+		if(instSp >= 0 && sp == instSp) {
+			if(S.activeInstances == 1) { done = true; return; }
+			to_world(S);
+		}
+		if(sp == 0) { done = true; return; }
+		const uint2 e = stack.get(--sp);
+		if(e.y > PRIM_BITS) { ngBase = e.x; ngMask = e.y; }
+		else { pgBase = e.x; pgHits = e.y; }
+	}
+
 	template < bool ALPHA, class Stack, class C >
 	MBD bool step_impl(const DScene& S, C& cnt, Stack& stack) {
 		if(done) return true;
 		if(--steps < 0) { ++cnt.errors; done = true; return true; }
-		if(instSp < 0 && pgHits) {
-			// instance leaves of the top level: enter one, keep the rest
-			uint32_t id = S.validInstance;
-			if(S.activeInstances != 1) {
-				const uint32_t j = 31u - uint32_t(__clz(int(pgHits)));
-				id = uint32_t(__ldg(S.tlasWidePrims + pgBase + j));
-				pgHits ^= 1u << j;
-				if(sp + 2 > WIDE_STACK) { ++cnt.errors; done = true; return true; }
-				if(ngMask > PRIM_BITS) stack.put(sp++, make_uint2(ngBase, ngMask));
-				if(pgHits) stack.put(sp++, make_uint2(pgBase, pgHits));
-			}
-			enter(S, id, cnt);
-		}
-		if(ngMask > PRIM_BITS) {
-			const uint32_t k = 31u - uint32_t(__clz(int(ngMask))); // highest bit first: nearest octant first
-			const uint32_t s = (k ^ oct) & 7u;
-			const uint32_t child = ngBase + uint32_t(__popc(ngMask & ((1u << s) - 1u)));
-			ngMask ^= 1u << k;
-			if(ngMask > PRIM_BITS) {
-				if(sp >= WIDE_STACK) { ++cnt.errors; done = true; return true; }
-				stack.put(sp++, make_uint2(ngBase, ngMask));
-			}
-			++cnt.nodes;
-			const float tmaxBox = t * scale * BOX_SLACK;
-			wide_node_test(nodes, child, o, inv, oct, tmaxBox, ngBase, ngMask, pgBase, pgHits);
-		}
-		if(instSp >= 0 && pgHits) {
-			do {
-				const uint32_t j = 31u - uint32_t(__clz(int(pgHits)));
-				pgHits ^= 1u << j;
-				// all three rows at once (every primitive has them), so a
-				// triangle costs one round trip to memory, not two
-				const float4* s4 = soup + 3 * size_t(pgBase + j);
-				const float4 a = __ldg(s4), b = __ldg(s4 + 1), c = __ldg(s4 + 2);
-				const int p = __float_as_int(a.w);
-				++cnt.prims;
-				float to;
-				f2 uv;
-				bool hit;
-				if(__float_as_int(b.w) == SOUP_TRIANGLE) {
-					hit = tri_test(o, kx, ky, kz, Sx, Sy, Sz, f4to3(a), f4to3(b), f4to3(c), to, uv) && to > 0.0f;
-					if(ALPHA && hit) hit = !alpha_cuts_triangle(alpha_ctx(S), lod(S), p, uv);
-				} else {
-					const PrimHit ph = ALPHA ? other_prim_test_alpha(&lod(S), o, d, p, alpha_ctx(S)) : other_prim_test(&lod(S), o, d, p);
-					hit = ph.hit; to = ph.t; uv = ph.uv;
-				}
-				if(hit) {
-					if(any) {
-						if(to < t * scale) { hitInst = inst; done = true; return true; }
+		if(instSp < 0 && pgHits) enter_pending(S, cnt, stack);
+		if(!done && ngMask > PRIM_BITS) visit_node(cnt, stack);
+		if(instSp >= 0) while(pgHits && !done) test_prim<ALPHA>(S, cnt, stack);
+		if(!done && ngMask <= PRIM_BITS && !pgHits) pop(S, stack);
+		return done;
+	}
+
+	// One step of every ray of the warp whose lane passes active, called by
+	// all 32 lanes together. Every lane's ray waits to enter an instance, to
+	// test primitives or to visit a node; the warp does the one that most of
+	// its rays wait for, an instance or a primitive counting more than a node
+	// so that their results, which shorten the other visits, do not come late.
+	// Rays thus collect until a part runs with many lanes. (One step of all
+	// three parts a pass ran the node test at 14 and the others at 2-5 lanes;
+	// without the votes the compiler besides threads a ray that entered an
+	// instance into a copy of the node test of its own, and the lanes drift
+	// apart.) ncu, incoherent bounces: 12.9 of 32 lanes per instruction against
+	// 9.0 (icosphere, 540p) and, with 38 % fewer instructions, against 5.6 to 9.9
+	// (4 096 instances, 360p) for steps without and with a meeting of the lanes
+	// between the parts. Weights: instances 3 and primitives 2 measured 10.3 ms
+	// of trace per 720p iteration of the instanced scene, 2 and 2 10.7, 1 and 1
+	// 11.7, 2 and 3 10.5, no votes 13.1; the icosphere is within 2 % for all.
+	template < class Stack, class C >
+	MBD bool warp_step(const DScene& S, C& cnt, Stack& stack, bool active) {
+		constexpr int INSTANCE_WEIGHT = 3, PRIM_WEIGHT = 2;
+		const bool go = active && !done;
+		const bool top = go && instSp < 0 && pgHits, prim = go && instSp >= 0 && pgHits, node = go && !pgHits;
+		const int wt = INSTANCE_WEIGHT * __popc(__ballot_sync(0xffffffffu, top));
+		const int wp = PRIM_WEIGHT * __popc(__ballot_sync(0xffffffffu, prim));
+		const int wn = __popc(__ballot_sync(0xffffffffu, node));
+		bool ran = false;
+		if(wt > wn && wt >= wp) {
+			if(top) { enter_pending(S, cnt, stack); ran = true; }
+		} else if(wp > wn) {
+			if(prim) {
+				ran = true;
+				do {
+					if constexpr(AM == ALPHA_SCENE) {
+						if(S.hasAlpha) test_prim<true>(S, cnt, stack);
+						else test_prim<false>(S, cnt, stack);
 					} else {
-						const float tw = __fdiv_rn(to, scale);
-						// better(): with no hit yet (hitInst -1) equal distances do not count
-						if(tw < t || (tw == t && (inst < hitInst || (inst == hitInst && p < hitPrim)))) {
-							t = tw; hitInst = inst; hitPrim = p; sp2 = uv;
-						}
+						test_prim<AM == ALPHA_ALWAYS>(S, cnt, stack);
 					}
-				}
-			} while(pgHits);
-		}
-		if(ngMask <= PRIM_BITS && !pgHits) {
-			if(instSp >= 0 && sp == instSp) {
-				if(S.activeInstances == 1) { done = true; return true; }
-				to_world(S);
+				} while(pgHits && !done);
 			}
-			if(sp == 0) { done = true; return true; }
-			const uint2 e = stack.get(--sp);
-			if(e.y > PRIM_BITS) { ngBase = e.x; ngMask = e.y; }
-			else { pgBase = e.x; pgHits = e.y; }
+		} else if(node) {
+			ran = true;
+			if(--steps < 0) { ++cnt.errors; done = true; }
+			else visit_node(cnt, stack);
 		}
-		return false;
+		__syncwarp();
+		if(ran && !done && ngMask <= PRIM_BITS && !pgHits) pop(S, stack);
+		return active && done;
 	}
 
 	MBD const DLod& lod(const DScene& S) const { return S.lods[__ldg(S.instanceLod + inst)]; }
@@ -380,9 +459,9 @@ template < int AM = ALPHA_SCENE, class Stack, class C >
 MBD HitRec closest_hit_wide(const DScene& S, f3 o, f3 dir, float tmax, C& cnt, Stack& stack) {
 	++cnt.rays;
 	WideTracerT<AM> t;
-	t.init(S, o, dir, tmax, false, cnt);
+	t.init(S, o, dir, tmax, false, stack);
 	while(!t.step(S, cnt, stack)) {}
-	return t.hit();
+	return t.hit(stack);
 }
 
 // Occlusion of a prepared shadow ray (origin offset, unit direction, length tmax).
@@ -390,9 +469,9 @@ template < class Stack, class C >
 MBD bool occluded_wide(const DScene& S, f3 a, f3 dir, float tmax, C& cnt, Stack& stack) {
 	++cnt.rays; ++cnt.shadow;
 	WideTracerT<ALPHA_SCENE> t;
-	t.init(S, a, dir, tmax, true, cnt);
+	t.init(S, a, dir, tmax, true, stack);
 	while(!t.step(S, cnt, stack)) {}
-	return t.occluded();
+	return t.occluded;
 }
 
 } // namespace mb
