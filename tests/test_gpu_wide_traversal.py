@@ -51,8 +51,8 @@ def _spec(n, instances, offset, seed):
                             (0.0, 1.0, 0.0), math.radians(40.0), 16, 16, name="wide_shapes")
 
 
-@pytest.mark.parametrize("instances", [1, 2, 9])
-@pytest.mark.parametrize("n", [1, 2, 3, 4, 8, 9, 24, 25, 300])
+@pytest.mark.parametrize("instances", [1, 2, 8, 9, 70])
+@pytest.mark.parametrize("n", [1, 2, 3, 4, 8, 9, 24, 25, 64, 65, 300])
 @pytest.mark.parametrize("offset", [0.0, 700.0])
 def test_hits_and_occlusion_bit_exact(dll, oracle, n, instances, offset):
     off = np.array([offset, -0.7 * offset, 0.3 * offset])
@@ -84,3 +84,15 @@ def test_hits_and_occlusion_bit_exact(dll, oracle, n, instances, offset):
         assert (gi >= 0).any()
     a, b = org.astype(np.float32), (org + d * rng.uniform(0.5, 2.0, (m, 1)) * np.linalg.norm(tgt - org, axis=1, keepdims=True)).astype(np.float32)
     assert np.array_equal(dll.trace_occlusion(a, b), sc.trace_any(a, b))
+
+
+# either side of the single-block sort's capacity, few distinct keys and many
+@pytest.mark.parametrize("distinct", [3, 1 << 60])
+@pytest.mark.parametrize("n", [31, 257, 2047, 2048, 2049])
+def test_short_sorts_are_stable(dll, n, distinct):
+    rng = np.random.default_rng(n)
+    k = rng.integers(0, distinct, n, dtype=np.uint64)
+    v = np.arange(n, dtype=np.int32)
+    gk, gv = bindings.sort_pairs(dll, k, v)
+    order = np.argsort(k, kind="stable")
+    assert np.array_equal(gk, k[order]) and np.array_equal(gv, v[order])
