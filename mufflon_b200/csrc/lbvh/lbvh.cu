@@ -699,7 +699,7 @@ cudaError_t LbvhBuilder::build_common(int mode, const LodBuildInput* lod, const 
 	if((e = reserve(numPrimitives)) != cudaSuccess) return e;
 	const bool wide = withSoup || mode == MODE_SCENE;
 	if(wide) {
-		const size_t wcap = wide_node_capacity(std::max<uint32_t>(used, 2u), mode == MODE_SCENE ? WIDE_TLAS_LEAF_MAX : WIDE_LEAF_MAX);
+		const size_t wcap = wide_node_capacity(std::max<uint32_t>(used, 2u), mode == MODE_SCENE ? WIDE_TLAS_LEAF_MAX : wide_leaf_max(used));
 		if(out.wideCapacity < wcap) {
 			if(out.wnodes) cudaFree(out.wnodes);
 			out.wnodes = nullptr;
@@ -784,7 +784,7 @@ cudaError_t LbvhBuilder::build_common(int mode, const LodBuildInput* lod, const 
 		WideBuildArgs wa{};
 		wa.n = n;
 		wa.numInternal = numInternal;
-		wa.leafMax = mode == MODE_SCENE ? WIDE_TLAS_LEAF_MAX : WIDE_LEAF_MAX;
+		wa.leafMax = mode == MODE_SCENE ? WIDE_TLAS_LEAF_MAX : wide_leaf_max(used);
 		wa.children = m_children;
 		wa.ranges = m_ranges;
 		wa.nodeData = m_nodeData;
