@@ -44,9 +44,9 @@ constexpr int SOUP_TRIANGLE = 1;
 
 struct alignas(16) WideNode {
 	float p[3];            // grid origin
-	uint32_t eimask;       // biased exponents ex | ey << 8 | ez << 16, mask of the slots in the children's block << 24
-	uint32_t childBase;    // index of the first child of the children's block
-	uint32_t primBase;     // first slot of this node's leaf primitives; instance level: mask of the instance slots
+	uint32_t eimask;       // biased exponents ex | ey << 8 | ez << 16, internal-slot mask << 24
+	uint32_t childBase;    // index of the first internal child
+	uint32_t primBase;     // first slot of this node's leaf primitives
 	uint32_t meta[2];      // per slot (unary count << 5) | offset, (1 << 5) | (24 + slot) internal, 0 empty
 	uint32_t qlo[3][2];    // per axis, 8 slots of 8 bits
 	uint32_t qhi[3][2];
@@ -67,12 +67,10 @@ struct WideBuildArgs {
 	const float4* nodeData;         // 2 per binary node: min.xyz, max.xyz (exact boxes)
 	const int32_t* sortedIds;       // sorted leaf index -> primitive / instance id
 	WideNode* nodes;                // capacity wide_node_capacity(n, leafMax)
-	int32_t* prims;                 // n: wide leaf slot -> primitive id; instance level: per node, its instance id or -1
-	bool instances;                 // the instance level: instances are children
-	uint32_t nodeCapacity;          // nodes (instance level: and instances)
-	uint32_t queueCapacity;
+	int32_t* prims;                 // n: wide leaf slot -> primitive / instance id
+	uint32_t nodeCapacity;
 	uint32_t* counters;             // device scratch, WIDE_COUNTERS entries
-	int2* queueA;                   // device scratch, queueCapacity entries each
+	int2* queueA;                   // device scratch, nodeCapacity entries each
 	int2* queueB;
 };
 constexpr int WIDE_COUNTERS = 8;
