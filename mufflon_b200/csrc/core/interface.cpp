@@ -151,6 +151,8 @@ void ensure_render_buffers(MufflonInstance& I) {
 	CHECK_CUDA(cudaMalloc(&r.hitId, n * 2 * sizeof(float)));
 	CHECK_CUDA(cudaMalloc(&r.workCounter, sizeof(unsigned int)));
 	CHECK_CUDA(cudaMalloc(&r.counters, 2 * sizeof(TraceCounters)));
+	CHECK_CUDA(cudaMalloc(&r.dIteration, sizeof(int32_t)));
+	CHECK_CUDA(cudaMallocHost(reinterpret_cast<void**>(&r.link), sizeof(RendererState::HostLink)));
 	CHECK_CUDA(cudaEventCreate(&r.evStart));
 	CHECK_CUDA(cudaEventCreate(&r.evStop));
 	r.needsReset = true;
@@ -345,9 +347,9 @@ void iterate_lt(MufflonInstance& I) {
 		CHECK_CUDA(launch_lt(S, r.ltParams, t, r.workCounter, r.counters, I.stream, r.ltMegakernel ? nullptr : r.ltWavefront));
 	}
 	CHECK_CUDA(cudaEventRecord(r.evStop, I.stream));
-	TraceCounters c{};
-	CHECK_CUDA(cudaMemcpyAsync(&c, r.counters, sizeof(TraceCounters), cudaMemcpyDeviceToHost, I.stream));
+	CHECK_CUDA(cudaMemcpyAsync(r.link->counters, r.counters, sizeof(TraceCounters), cudaMemcpyDeviceToHost, I.stream));
 	CHECK_CUDA(cudaStreamSynchronize(I.stream));
+	const TraceCounters c = r.link->counters[0];
 	CHECK_CUDA(cudaEventElapsedTime(&r.lastKernelMs, r.evStart, r.evStop));
 	r.lastCounters = c;
 	r.lastExtend = TraceCounters{};
@@ -395,8 +397,8 @@ void RendererState::release() {
 	graphExec = nullptr;
 	graphKey.clear();
 	if(dIteration) cudaFree(dIteration);
-	if(hIteration) cudaFreeHost(hIteration);
-	dIteration = nullptr; hIteration = nullptr;
+	if(link) cudaFreeHost(link);
+	dIteration = nullptr; link = nullptr;
 	if(wfMemory) cudaFree(wfMemory);
 	wfMemory = nullptr;
 	wf = WfState{};
@@ -428,8 +430,23 @@ void RendererState::release() {
 	evStart = evStop = nullptr;
 	width = height = 0;
 }
+cudaError_t CallScratch::reserve(size_t need) {
+	if(need <= bytes) return cudaSuccess;
+	release();
+	const cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&device), need);
+	if(e != cudaSuccess) { device = nullptr; return e; }
+	bytes = need;
+	return cudaSuccess;
+}
+void CallScratch::trim() { if(bytes > KEEP) release(); }
+void CallScratch::release() {
+	cudaFree(device);
+	device = nullptr;
+	bytes = 0;
+}
 MufflonInstance::~MufflonInstance() {
 	renderer.release();
+	scratch.release();
 	scene.release();
 	if(stream) cudaStreamDestroy(stream);
 }
@@ -1416,10 +1433,6 @@ Boolean render_iterate(MufflonInstanceHdl h, ProcessTime* iterTime, ProcessTime*
 		// (the iteration number is read from device memory), so it is
 		// captured once and replayed; it is captured again when anything it
 		// was built from changes.
-		if(!r.dIteration) {
-			CHECK_CUDA(cudaMalloc(&r.dIteration, sizeof(int32_t)));
-			CHECK_CUDA(cudaMallocHost(&r.hIteration, sizeof(int32_t)));
-		}
 		rs.dIteration = r.dIteration;
 		rs.iteration = 0; // read from dIteration: not part of the captured launches
 		std::vector<unsigned char> key;
@@ -1444,8 +1457,8 @@ Boolean render_iterate(MufflonInstanceHdl h, ProcessTime* iterTime, ProcessTime*
 			r.graphKey = key;
 			r.graphLaunches = info.launches;
 		}
-		*r.hIteration = r.iteration;
-		CHECK_CUDA(cudaMemcpyAsync(r.dIteration, r.hIteration, sizeof(int32_t), cudaMemcpyHostToDevice, I.stream));
+		r.link->iteration = r.iteration;
+		CHECK_CUDA(cudaMemcpyAsync(r.dIteration, &r.link->iteration, sizeof(int32_t), cudaMemcpyHostToDevice, I.stream));
 		CHECK_CUDA(cudaEventRecord(r.evStart, I.stream));
 		CHECK_CUDA(cudaGraphLaunch(r.graphExec, I.stream));
 		info.launches = r.graphLaunches;
@@ -1455,12 +1468,12 @@ Boolean render_iterate(MufflonInstanceHdl h, ProcessTime* iterTime, ProcessTime*
 		else CHECK_CUDA(launch_pt_wavefront(I.scene.desc, r.params, rs, r.wf, r.counters, I.stream, &info, tune));
 	}
 	CHECK_CUDA(cudaEventRecord(r.evStop, I.stream));
-	TraceCounters both[2];
-	CHECK_CUDA(cudaMemcpyAsync(both, r.counters, 2 * sizeof(TraceCounters), cudaMemcpyDeviceToHost, I.stream));
-	unsigned bounceQueue[WF_BOUNCE_STATS] = {};
+	const TraceCounters* both = r.link->counters;
+	CHECK_CUDA(cudaMemcpyAsync(r.link->counters, r.counters, 2 * sizeof(TraceCounters), cudaMemcpyDeviceToHost, I.stream));
+	const unsigned* bounceQueue = r.link->bounceQueue;
 	if(!r.megakernel)
-		CHECK_CUDA(cudaMemcpyAsync(bounceQueue, r.wf.counters + WF_COUNTERS - WF_BOUNCE_STATS, sizeof(bounceQueue),
-		                           cudaMemcpyDeviceToHost, I.stream));
+		CHECK_CUDA(cudaMemcpyAsync(r.link->bounceQueue, r.wf.counters + WF_COUNTERS - WF_BOUNCE_STATS,
+		                           sizeof(r.link->bounceQueue), cudaMemcpyDeviceToHost, I.stream));
 	CHECK_CUDA(cudaStreamSynchronize(I.stream));
 	if(!r.megakernel) {
 		// next iteration's plan: the first bounce >= wavefrontBounces whose
@@ -1990,13 +2003,8 @@ static void run_adjoint(MufflonInstance& I, uint32_t spp, const float* imageGrad
 	desc.maxSteps = step_limit(r);
 	desc.camera.resX = uint16_t(w);
 	desc.camera.resY = uint16_t(hgt);
-	uint64_t* rng = nullptr;
-	float *dImg = nullptr, *dGrad = nullptr, *dEmis = nullptr;
-	unsigned char* dTarget = nullptr;
-	void* adjMem = nullptr;
 	cudaEvent_t a = nullptr, b = nullptr;
 	auto cleanup = [&]() {
-		cudaFree(rng); cudaFree(dImg); cudaFree(dGrad); cudaFree(dEmis); cudaFree(dTarget); cudaFree(adjMem);
 		if(a) cudaEventDestroy(a);
 		if(b) cudaEventDestroy(b);
 	};
@@ -2006,19 +2014,27 @@ static void run_adjoint(MufflonInstance& I, uint32_t spp, const float* imageGrad
 		ensure_wavefront_buffers(I);
 	}
 	try {
-		if(wavefront) CHECK_CUDA(cudaMalloc(&adjMem, adjoint_bytes(n, r.params.maxPathLength)));
-		CHECK_CUDA(cudaMalloc(&rng, n * 8));
-		CHECK_CUDA(cudaMalloc(&dImg, n * 12));
+		// one slab of the kept scratch memory: the replay's bookkeeping,
+		// generators, image gradient, texel gradient, emission gradient and flags
+		const size_t adjBytes = wavefront ? align256(adjoint_bytes(n, r.params.maxPathLength)) : 0;
+		const size_t gradBytes = texIndex >= 0 ? align256(nt * 12) : 0;
+		const size_t flagBytes = emitTarget ? align256(emitTarget->size()) : 0;
+		CHECK_CUDA(I.scratch.reserve(adjBytes + align256(n * 8) + align256(n * 12) + gradBytes + 256 + flagBytes));
+		char* m = I.scratch.device;
+		auto take = [&](size_t bytes) { char* p = m; m += bytes; return p; };
+		void* adjMem = take(adjBytes);
+		uint64_t* rng = reinterpret_cast<uint64_t*>(take(align256(n * 8)));
+		float* dImg = reinterpret_cast<float*>(take(align256(n * 12)));
+		float* dGrad = reinterpret_cast<float*>(take(gradBytes));
+		float* dEmis = reinterpret_cast<float*>(take(256));
+		unsigned char* dTarget = reinterpret_cast<unsigned char*>(take(flagBytes));
 		AdjointTargets T;
 		if(texIndex >= 0) {
-			CHECK_CUDA(cudaMalloc(&dGrad, nt * 12));
 			CHECK_CUDA(cudaMemsetAsync(dGrad, 0, nt * 12, I.stream));
 			T.texIndex = texIndex;
 			T.texGrad = dGrad;
 		}
 		if(emitTarget) {
-			CHECK_CUDA(cudaMalloc(&dEmis, 12));
-			CHECK_CUDA(cudaMalloc(&dTarget, emitTarget->size()));
 			CHECK_CUDA(cudaMemsetAsync(dEmis, 0, 12, I.stream));
 			CHECK_CUDA(cudaMemcpyAsync(dTarget, emitTarget->data(), emitTarget->size(), cudaMemcpyHostToDevice, I.stream));
 			T.emitTarget = dTarget;
@@ -2051,6 +2067,7 @@ static void run_adjoint(MufflonInstance& I, uint32_t spp, const float* imageGrad
 		TraceCounters tc[2] = {};
 		if(wavefront) CHECK_CUDA(cudaMemcpyAsync(tc, r.counters, sizeof(tc), cudaMemcpyDeviceToHost, I.stream));
 		CHECK_CUDA(cudaStreamSynchronize(I.stream));
+		I.scratch.trim();
 		if(deviceMs) CHECK_CUDA(cudaEventElapsedTime(deviceMs, a, b));
 		check_traversal(tc[0].errors + tc[1].errors, desc.maxSteps);
 	} catch(...) {
@@ -2164,24 +2181,27 @@ Boolean mufflon_trace_rays(MufflonInstanceHdl h, const float* rays, const float*
 	CHECK(rays && t && inst && prim, "invalid arguments");
 	load_scene_if_needed(I);
 	if(n == 0) return true;
-	float *dr = nullptr, *dg = nullptr, *dt = nullptr, *dsp = nullptr;
-	int32_t *di = nullptr, *dp = nullptr;
-	CHECK_CUDA(cudaMalloc(&dr, size_t(n) * 24));
-	CHECK_CUDA(cudaMalloc(&dt, size_t(n) * 4));
-	CHECK_CUDA(cudaMalloc(&di, size_t(n) * 4));
-	CHECK_CUDA(cudaMalloc(&dp, size_t(n) * 4));
-	CHECK_CUDA(cudaMalloc(&dsp, size_t(n) * 8));
-	if(geo) CHECK_CUDA(cudaMalloc(&dg, size_t(n) * 12));
-	CHECK_CUDA(cudaMemcpyAsync(dr, rays, size_t(n) * 24, cudaMemcpyHostToDevice, I.stream));
-	if(geo) CHECK_CUDA(cudaMemcpyAsync(dg, geo, size_t(n) * 12, cudaMemcpyHostToDevice, I.stream));
+	const size_t N = n;
+	auto part = [](size_t bytes) { return align256(bytes); };
+	CHECK_CUDA(I.scratch.reserve(part(N * 24) + 3 * part(N * 4) + part(N * 8) + (geo ? N * 12 : 0)));
+	char* m = I.scratch.device;
+	auto take = [&](size_t bytes) { char* p = m; m += part(bytes); return p; };
+	float* dr = reinterpret_cast<float*>(take(N * 24));
+	float* dt = reinterpret_cast<float*>(take(N * 4));
+	int32_t* di = reinterpret_cast<int32_t*>(take(N * 4));
+	int32_t* dp = reinterpret_cast<int32_t*>(take(N * 4));
+	float* dsp = reinterpret_cast<float*>(take(N * 8));
+	float* dg = geo ? reinterpret_cast<float*>(m) : nullptr;
+	CHECK_CUDA(cudaMemcpyAsync(dr, rays, N * 24, cudaMemcpyHostToDevice, I.stream));
+	if(geo) CHECK_CUDA(cudaMemcpyAsync(dg, geo, N * 12, cudaMemcpyHostToDevice, I.stream));
 	if(I.renderer.megakernel) CHECK_CUDA(launch_trace_rays(I.scene.desc, dr, dg, tmax, n, dt, di, dp, dsp, I.stream));
 	else CHECK_CUDA(launch_trace_rays_wide(I.scene.desc, dr, dg, tmax, n, dt, di, dp, dsp, I.stream));
-	CHECK_CUDA(cudaMemcpyAsync(t, dt, size_t(n) * 4, cudaMemcpyDeviceToHost, I.stream));
-	CHECK_CUDA(cudaMemcpyAsync(inst, di, size_t(n) * 4, cudaMemcpyDeviceToHost, I.stream));
-	CHECK_CUDA(cudaMemcpyAsync(prim, dp, size_t(n) * 4, cudaMemcpyDeviceToHost, I.stream));
-	if(sp) CHECK_CUDA(cudaMemcpyAsync(sp, dsp, size_t(n) * 8, cudaMemcpyDeviceToHost, I.stream));
+	CHECK_CUDA(cudaMemcpyAsync(t, dt, N * 4, cudaMemcpyDeviceToHost, I.stream));
+	CHECK_CUDA(cudaMemcpyAsync(inst, di, N * 4, cudaMemcpyDeviceToHost, I.stream));
+	CHECK_CUDA(cudaMemcpyAsync(prim, dp, N * 4, cudaMemcpyDeviceToHost, I.stream));
+	if(sp) CHECK_CUDA(cudaMemcpyAsync(sp, dsp, N * 8, cudaMemcpyDeviceToHost, I.stream));
 	CHECK_CUDA(cudaStreamSynchronize(I.stream));
-	cudaFree(dr); cudaFree(dg); cudaFree(dt); cudaFree(di); cudaFree(dp); cudaFree(dsp);
+	I.scratch.trim();
 	return true;
 	CATCH_ALL(false)
 }
@@ -2193,18 +2213,18 @@ Boolean mufflon_trace_occlusion(MufflonInstanceHdl h, const float* a, const floa
 	CHECK(a && b && occ, "invalid arguments");
 	load_scene_if_needed(I);
 	if(n == 0) return true;
-	float *da = nullptr, *db = nullptr;
-	uint8_t* dout = nullptr;
-	CHECK_CUDA(cudaMalloc(&da, size_t(n) * 12));
-	CHECK_CUDA(cudaMalloc(&db, size_t(n) * 12));
-	CHECK_CUDA(cudaMalloc(&dout, n));
+	const size_t points = align256(size_t(n) * 12);
+	CHECK_CUDA(I.scratch.reserve(2 * points + n));
+	float* da = reinterpret_cast<float*>(I.scratch.device);
+	float* db = reinterpret_cast<float*>(I.scratch.device + points);
+	uint8_t* dout = reinterpret_cast<uint8_t*>(I.scratch.device + 2 * points);
 	CHECK_CUDA(cudaMemcpyAsync(da, a, size_t(n) * 12, cudaMemcpyHostToDevice, I.stream));
 	CHECK_CUDA(cudaMemcpyAsync(db, b, size_t(n) * 12, cudaMemcpyHostToDevice, I.stream));
 	if(I.renderer.megakernel) CHECK_CUDA(launch_occlusion(I.scene.desc, da, db, n, dout, I.stream));
 	else CHECK_CUDA(launch_occlusion_wide(I.scene.desc, da, db, n, dout, I.stream));
 	CHECK_CUDA(cudaMemcpyAsync(occ, dout, n, cudaMemcpyDeviceToHost, I.stream));
 	CHECK_CUDA(cudaStreamSynchronize(I.stream));
-	cudaFree(da); cudaFree(db); cudaFree(dout);
+	I.scratch.trim();
 	return true;
 	CATCH_ALL(false)
 }
