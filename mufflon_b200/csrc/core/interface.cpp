@@ -448,6 +448,8 @@ MufflonInstance::~MufflonInstance() {
 	renderer.release();
 	scratch.release();
 	scene.release();
+	if(copyEvent) cudaEventDestroy(copyEvent);
+	if(copyStream) cudaStreamDestroy(copyStream);
 	if(stream) cudaStreamDestroy(stream);
 }
 } // namespace mb

@@ -322,6 +322,8 @@ struct MufflonInstance {
 	std::recursive_mutex iterationMutex;
 	int device = 0;
 	cudaStream_t stream = nullptr;
+	cudaStream_t copyStream = nullptr; // uploads beside the hierarchy builds (scene_build.cpp)
+	cudaEvent_t copyEvent = nullptr;
 	std::vector<std::unique_ptr<HostObject>> objects;
 	std::vector<std::unique_ptr<HostInstance>> instances;
 	std::vector<std::unique_ptr<HostMaterial>> materials;

@@ -147,11 +147,49 @@ MBD float surface(f3 mn, f3 mx) {
 }
 
 // ---------------------------------------------------------------- Morton
+// Bounds of an object: block partial minima and maxima into six ordered keys
+// (unsigned order = float order), decoded by the last launch. NaN coordinates
+// are passed over, as on the host.
+MBD uint32_t ordered_key(float x) {
+	const uint32_t u = __float_as_uint(x);
+	return u ^ (u >> 31 ? 0xFFFFFFFFu : 0x80000000u);
+}
+__global__ void k_box_init(uint32_t* keys) {
+	if(threadIdx.x < 6) keys[threadIdx.x] = ordered_key(threadIdx.x < 3 ? FLT_MAX : -FLT_MAX);
+}
+__global__ void __launch_bounds__(256) k_box_reduce(const float* __restrict__ vertices, uint32_t numVertices,
+                                                    const float4* __restrict__ spheres, uint32_t numSpheres, uint32_t* keys) {
+	float mn[3] = { FLT_MAX, FLT_MAX, FLT_MAX }, mx[3] = { -FLT_MAX, -FLT_MAX, -FLT_MAX };
+	auto add = [&](int a, float lo, float hi) {
+		mn[a] = lo < mn[a] ? lo : mn[a];
+		mx[a] = hi > mx[a] ? hi : mx[a];
+	};
+	const uint32_t step = gridDim.x * blockDim.x, first = blockIdx.x * blockDim.x + threadIdx.x;
+	for(uint32_t i = first; i < numVertices; i += step)
+		for(int a = 0; a < 3; ++a) { const float x = vertices[3 * size_t(i) + a]; add(a, x, x); }
+	for(uint32_t i = first; i < numSpheres; i += step) {
+		const float4 s = spheres[i];
+		add(0, s.x - s.w, s.x + s.w); add(1, s.y - s.w, s.y + s.w); add(2, s.z - s.w, s.z + s.w);
+	}
+	for(int a = 0; a < 3; ++a) {
+		const uint32_t lo = __reduce_min_sync(0xffffffffu, ordered_key(mn[a]));
+		const uint32_t hi = __reduce_max_sync(0xffffffffu, ordered_key(mx[a]));
+		if((threadIdx.x & 31u) == 0) { atomicMin(keys + a, lo); atomicMax(keys + 3 + a, hi); }
+	}
+}
+__global__ void k_box_final(uint32_t* keys) {
+	if(threadIdx.x >= 6) return;
+	const uint32_t k = keys[threadIdx.x];
+	keys[8 + threadIdx.x] = k ^ (k >> 31 ? 0x80000000u : 0xFFFFFFFFu);
+}
+
 __global__ void k_morton_lod(LodBuildInput in, uint32_t n, u64* keys, int32_t* vals, int bits) {
 	const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
 	if(i >= n) return;
 	const f3 c = lod_centroid(in, int(i));
-	keys[i] = bits == 30 ? morton30(c, in.aabbMin, in.aabbMax) : morton63(c, in.aabbMin, in.aabbMax);
+	const float* mn = in.deviceBox ? in.deviceBox : in.aabbMin;
+	const float* mx = in.deviceBox ? in.deviceBox + 3 : in.aabbMax;
+	keys[i] = bits == 30 ? morton30(c, mn, mx) : morton63(c, mn, mx);
 	vals[i] = int32_t(i);
 }
 
@@ -594,6 +632,8 @@ LbvhBuilder::~LbvhBuilder() {
 	cudaFree(m_tileCounter); cudaFree(m_error);
 	cudaFree(m_ranges); cudaFree(m_wideCounters); cudaFree(m_wideQueueA); cudaFree(m_wideQueueB);
 	if(m_hostCount) cudaFreeHost(m_hostCount);
+	if(m_hostBox) cudaFreeHost(m_hostBox);
+	cudaFree(m_boxKeys);
 	for(auto& e : m_ev) if(e) cudaEventDestroy(e);
 	for(auto& e : m_wideEv) if(e) cudaEventDestroy(e);
 	if(m_fork) cudaEventDestroy(m_fork);
@@ -823,6 +863,27 @@ cudaError_t LbvhBuilder::build_common(int mode, const LodBuildInput* lod, const 
 		m_times = { t[0], t[1], t[2], t[3], t[4], t[5], t[6], t[7], t[8] };
 	}
 	return cudaSuccess;
+}
+
+cudaError_t LbvhBuilder::measure_box(LodBuildInput& in, uint32_t numVertices, cudaStream_t stream) {
+	cudaError_t e;
+	if(!m_boxKeys) {
+		if((e = cudaMallocHost(&m_hostBox, 6 * sizeof(float))) != cudaSuccess) return e;
+		if((e = cudaMalloc(&m_boxKeys, 16 * sizeof(uint32_t))) != cudaSuccess) return e;
+	}
+	k_box_init<<<1, 32, 0, stream>>>(m_boxKeys);
+	k_box_reduce<<<std::min(blocks_for(std::max(numVertices, in.numSpheres), 256), 148u * 4u), 256, 0, stream>>>(
+		in.vertices, numVertices, in.spheres, in.numSpheres, m_boxKeys);
+	k_box_final<<<1, 32, 0, stream>>>(m_boxKeys);
+	in.deviceBox = reinterpret_cast<const float*>(m_boxKeys + 8);
+	if((e = cudaMemcpyAsync(m_hostBox, m_boxKeys + 8, 6 * sizeof(float), cudaMemcpyDeviceToHost, stream)) != cudaSuccess) return e;
+	return cudaGetLastError();
+}
+
+cudaError_t LbvhBuilder::read_box(float mn[3], float mx[3], cudaStream_t stream) {
+	const cudaError_t e = cudaStreamSynchronize(stream);
+	for(int a = 0; a < 3; ++a) { mn[a] = m_hostBox[a]; mx[a] = m_hostBox[3 + a]; }
+	return e;
 }
 
 cudaError_t LbvhBuilder::build_lod(const LodBuildInput& in, BvhBuffers& out, cudaStream_t stream, bool withSoup) {

@@ -30,6 +30,7 @@ struct LodBuildInput {
 	const uint32_t* indices; // device, 3 per triangle then 4 per quad
 	const float4* spheres;   // device
 	float aabbMin[3], aabbMax[3];
+	const float* deviceBox;  // device, min xyz, max xyz: used in place of aabbMin and aabbMax where set (measure_box)
 };
 
 struct SceneBuildInput {
@@ -76,6 +77,10 @@ public:
 	// Builds into `out` (grown as needed). Returns cudaSuccess or the first
 	// CUDA error; a failed bounded wait inside the sort is reported as
 	// cudaErrorLaunchTimeout.
+	// The bounds of an object's vertices and spheres, on the device for the
+	// build that follows (in.deviceBox), and read_box for the host after it.
+	cudaError_t measure_box(LodBuildInput& in, uint32_t numVertices, cudaStream_t stream);
+	cudaError_t read_box(float mn[3], float mx[3], cudaStream_t stream);
 	cudaError_t build_lod(const LodBuildInput& in, BvhBuffers& out, cudaStream_t stream, bool withSoup = true);
 	cudaError_t build_scene(const SceneBuildInput& in, BvhBuffers& out, cudaStream_t stream);
 
@@ -124,6 +129,8 @@ private:
 	unsigned int* m_tileCounter = nullptr; // 8
 	unsigned int* m_error = nullptr;
 	int32_t* m_hostCount = nullptr;   // pinned
+	uint32_t* m_boxKeys = nullptr;    // 6 ordered keys, then the box they decode to
+	float* m_hostBox = nullptr;       // pinned, 6
 	int32_t m_lastN = 0;
 	bool m_timing = false;
 	int m_mortonBits = 63;

@@ -40,3 +40,29 @@ def test_mixed_calls(core_lib_path):
         assert np.abs(g0 - g1).max() <= 2400 * 2.0 ** -24 * max(np.abs(g1).max(), 1e-30)
         used.render_reset()
         used.render_iterate()
+
+
+# around the size from which bounds are taken on the device; spheres beyond the vertices; exact zeros, whose sign
+# the host's order decides
+@pytest.mark.parametrize("n", [8000, 8192, 9001, 40000])
+@pytest.mark.parametrize("zeros", [False, True])
+def test_device_bounds(dll, n, zeros):
+    rng = np.random.default_rng(n)
+    nt = n // 3
+    v = rng.uniform(-3.0, 5.0, (3 * nt, 3)).astype(np.float32)
+    if zeros:
+        v = np.abs(v)
+        v[rng.integers(0, len(v), 40), 1] = np.where(rng.uniform(size=40) < 0.5, np.float32(0.0), np.float32(-0.0))
+    sph = np.concatenate([rng.uniform(0.5, 6.0, (n - 3 * nt + 50, 3)), rng.uniform(0.01, 0.4, (n - 3 * nt + 50, 1))], 1).astype(np.float32)
+    lod = scenes.LodSpec(v, np.tile(np.array([0, 0, 1], np.float32), (len(v), 1)), np.zeros((len(v), 2), np.float32),
+                         np.arange(3 * nt, dtype=np.uint32).reshape(nt, 3), np.zeros((0, 4), np.uint32), np.zeros(nt, np.uint16),
+                         sph, np.zeros(len(sph), np.uint16), name="cloud")
+    spec = scenes.SceneSpec([lod], np.array([scenes.identity34()], np.float32), np.zeros(1, np.uint32),
+                            [scenes.MaterialSpec(scenes.MAT_LAMBERT)], np.array([[0, 9, 0, 1, 1, 1]], np.float32), None,
+                            (0.0, 0.0, 9.0), (0.0, 0.0, -1.0), (0.0, 1.0, 0.0), 0.7, 16, 16, name="cloud")
+    dll.world_clear_all()
+    bindings.load_scene_spec(dll, spec)
+    nodes, prims, internal = dll.get_bvh(0)
+    _, _, want, want_prims, want_internal, _ = bindings.lbvh_build(dll, lod)  # with the host's bounds
+    assert internal == want_internal and np.array_equal(prims, want_prims)
+    assert np.array_equal(nodes.view(np.uint32), want.view(np.uint32))
