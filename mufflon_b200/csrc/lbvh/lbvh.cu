@@ -694,8 +694,8 @@ cudaError_t LbvhBuilder::sort_pairs(uint64_t* keys, int32_t* values, uint32_t n,
 	cudaMemsetAsync(m_hist, 0, 8 * 256 * sizeof(uint32_t), stream);
 	cudaMemsetAsync(m_tileCounter, 0, 8 * sizeof(unsigned int), stream);
 	const unsigned hb = std::min<unsigned>(blocks_for(n, 256), 148u * 8u);
-	k_sort_hist<<<hb, 256, 0, stream>>>(keys, n, m_hist);
-	k_sort_scan<<<8, 256, 0, stream>>>(m_hist);
+	k_sort_hist<<<hb, 256, 0, stream>>>(keys, n, m_hist, passes);
+	k_sort_scan<<<passes, 256, 0, stream>>>(m_hist);
 	u64* kin = keys; u64* kout = (keys == m_keysA) ? m_keysB : m_keysA;
 	int32_t* vin = values; int32_t* vout = (values == m_valsA) ? m_valsB : m_valsA;
 	// ping-pong between the caller's buffers and the builder's spare ones

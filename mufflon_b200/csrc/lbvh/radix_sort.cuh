@@ -24,17 +24,19 @@ constexpr size_t SORT_SMEM = size_t(SORT_TILE) * 8 + size_t(SORT_TILE) * 4 + siz
 constexpr unsigned SPIN_LIMIT = 1u << 22;
 
 // ---------------------------------------------------------------- radix sort
-__global__ void k_sort_hist(const u64* keys, uint32_t n, uint32_t* hist) {
+// Digit counts of the keys' low 8 * passes bits.
+__global__ void k_sort_hist(const u64* keys, uint32_t n, uint32_t* hist, int passes) {
 	__shared__ uint32_t h[8 * 256];
 	for(int i = threadIdx.x; i < 8 * 256; i += blockDim.x) h[i] = 0;
 	__syncthreads();
 	for(uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
 		const u64 k = keys[i];
 #pragma unroll
-		for(int p = 0; p < 8; ++p) atomicAdd(&h[p * 256 + ((k >> (8 * p)) & 255u)], 1u);
+		for(int p = 0; p < 8; ++p)
+			if(p < passes) atomicAdd(&h[p * 256 + ((k >> (8 * p)) & 255u)], 1u);
 	}
 	__syncthreads();
-	for(int i = threadIdx.x; i < 8 * 256; i += blockDim.x)
+	for(int i = threadIdx.x; i < passes * 256; i += blockDim.x)
 		if(h[i]) atomicAdd(&hist[i], h[i]);
 }
 

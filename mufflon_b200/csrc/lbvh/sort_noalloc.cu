@@ -97,7 +97,7 @@ cudaError_t sort_pairs_noalloc(uint64_t* keys, int32_t* values, uint32_t n, cuda
 	if((e = cudaMemsetAsync(counters, 0, 8 * sizeof(unsigned int), stream)) != cudaSuccess) return e;
 	if((e = cudaMemsetAsync(error, 0, sizeof(unsigned int), stream)) != cudaSuccess) return e;
 	const unsigned hb = std::min<unsigned>((n + 255) / 256, 148u * 8u);
-	k_sort_hist<<<hb, 256, 0, stream>>>(keys, n, hist);
+	k_sort_hist<<<hb, 256, 0, stream>>>(keys, n, hist, 8);
 	k_sort_scan<<<8, 256, 0, stream>>>(hist);
 	u64* kin = keys; u64* kout = spareKeys;
 	int32_t* vin = values; int32_t* vout = spareVals;

@@ -158,3 +158,21 @@ def test_vcm_in_the_registry():
         assert not d.renderer_set_parameter_float("Relative merge radius", 0.01)
     finally:
         d.close()
+
+
+# (width, height, path length, merge radius): fewer pixels than one block of the photon list (1 024), the last one
+# below, at and after its edge, and more blocks (1 027) than the scan of their counts takes at once (1 024); the
+# bucket counts (1.15 x pixels x path length) need 1, 2 and 3 passes of the 8-bit sort.
+@pytest.mark.parametrize("width,height,m,radius", [(1, 1, 2, 0.05), (31, 33, 3, 0.02), (32, 32, 3, 0.02), (41, 25, 3, 0.02),
+                                                   (1025, 1025, 2, 0.0008)])
+def test_vcm_photon_list_sizes_match_oracle(oracle, width, height, m, radius):
+    """The merges' sums follow the order of a bucket's photons, so they are the
+    oracle's bit for bit only if every photon is listed once and in order."""
+    spec = scenes.cornell_box(1, width=width, height=height)
+    params = {"Seed": 3, "Min. path length": 0, "Max. path length": m}
+    ob = oracle.OracleVcm(oracle.OracleScene(spec), seed=3, min_path=0, max_path=m, merge_radius=radius)
+    seen = []
+    out, stats = _gpu_vcm(spec, params, 1, radius, per_iteration=_compare(ob, seen, m))
+    assert width * height < 1000 or seen[0][1] > 10, seen
+    assert stats["errors"] == 0
+    assert _rel_rmse(out["Radiance"], ob.target("Radiance")) <= 1e-5
