@@ -349,7 +349,7 @@ __global__ void k_ltw_start(const DScene S, const LtParams P, const LtTargets T,
 
 // Generation gen: the segments of queue gen & 1 (closest hit) and the camera
 // connections counted in LTW_SH0 + (gen & 1) (any hit), taken by persistent
-// warps 32 items at a time once all their lanes are idle.
+// warps whenever enough of their lanes are idle (ray_queue.cuh).
 template < int AM >
 __global__ void __launch_bounds__(128, LTW_TRACE_BLOCKS) k_ltw_trace(const DScene S, const LtParams P, const LtTargets T, LtwState W,
                                                    int gen, TraceCounters* counters) {

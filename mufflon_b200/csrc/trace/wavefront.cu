@@ -3,10 +3,11 @@
 //
 //   camera   one thread per pixel: consume the camera's and the first walk's
 //            random numbers, write the primary ray into queue 0;
-//   extend   persistent warps pull 32 rays at a time from the current queue
-//            (one atomic per warp) and run closest-hit traversal only;
-//   shadow   persistent warps pull shadow-ray groups, run any-hit traversal
-//            and add the visible next-event contributions to the path's sum;
+//   trace    persistent warps refill their idle lanes from the current queue
+//            (one atomic per refill) and run traversal only: closest hit for
+//            the extension rays, any hit for the previous shade's shadow-ray
+//            groups, whose visible next-event contributions they add to the
+//            path's sum;
 //   shade    one thread per queued path: hit attributes, emission with MIS,
 //            then (if the path continues) next-event estimation, which
 //            appends shadow rays, and the BSDF sample, Russian roulette and
@@ -16,7 +17,7 @@
 // Each kernel is small and does one kind of work, so it keeps its lanes
 // converged, stays in the instruction cache and needs few registers. The
 // per-path order of random numbers and of radiance additions is the one of
-// pt_sample: the shadow kernel of bounce k runs after shade k and before
+// pt_sample: the shadow rays of bounce k are traced after shade k and before
 // shade k+1, so a next-event contribution is added between the emission terms
 // that surround it, exactly as the sequential loop adds them.
 #include "accumulate.cuh"
@@ -1172,6 +1173,13 @@ template < class SP > TraceKernel<SP> trace_kernel(int perSm, bool counting, boo
 	return table[c][idx];
 }
 
+// Resident blocks per SM the tail is compiled for. It holds a path's shading
+// state and its ray's traversal, and spilled some 250 bytes a thread with 4
+// blocks. Tail of an iteration with 5 / 4 / 3 / 2 blocks: 256 x 256 box 0.307 /
+// 0.271 / 0.261 / 0.248 ms, 64 x 64 box 0.147 / 0.134 / 0.131 / 0.140, 1080p
+// icosphere 0.539 / 0.462 / 0.442 / 0.433, cutouts 0.182 / 0.161 / 0.149 / 0.147.
+constexpr int TAIL_BLOCKS = 3;
+
 template < class SP > struct TailKernel {
 	using Fn = void (*)(const SP, WfState, int, int, int, TraceCounters*, int, unsigned, int);
 	Fn fn;
@@ -1179,8 +1187,9 @@ template < class SP > struct TailKernel {
 };
 template < class SP > TailKernel<SP> tail_kernel(bool counting, bool alpha) {
 	static TailKernel<SP> k[3] = {};
-	const typename TailKernel<SP>::Fn fn = counting ? k_tail<4, SP, LocalCounters, ALPHA_SCENE>
-	                                     : alpha ? k_tail<4, SP, NoCounters, ALPHA_ALWAYS> : k_tail<4, SP, NoCounters, ALPHA_NEVER>;
+	const typename TailKernel<SP>::Fn fn = counting ? k_tail<TAIL_BLOCKS, SP, LocalCounters, ALPHA_SCENE>
+	                                     : alpha ? k_tail<TAIL_BLOCKS, SP, NoCounters, ALPHA_ALWAYS>
+	                                             : k_tail<TAIL_BLOCKS, SP, NoCounters, ALPHA_NEVER>;
 	const int c = counting ? 2 : (alpha ? 1 : 0);
 	if(!k[c].fn) k[c] = { fn, persistent_blocks(reinterpret_cast<const void*>(fn), int(WF_BLOCK)) };
 	return k[c];
