@@ -29,10 +29,10 @@ PARAMS = {"megakernel": "Megakernel", "trace_blocks": "Trace blocks per SM",
 
 
 def default_candidates() -> List[Dict[str, int]]:
-    c = [dict(megakernel=0, trace_blocks=b, wavefront_bounces=k, refill_lanes=32, tail_paths=t)
+    c = [dict(megakernel=0, trace_blocks=b, wavefront_bounces=k, refill_lanes=12, tail_paths=t)
          for b, k, t in itertools.product((4, 6), (1, 2), (32768, 98304, 262144))]
-    c += [dict(megakernel=0, trace_blocks=6, wavefront_bounces=2, refill_lanes=32, tail_paths=98304, sort_bits=s)
-          for s in (0, 16)]
+    c += [dict(megakernel=0, trace_blocks=6, wavefront_bounces=2, refill_lanes=r, tail_paths=98304, sort_bits=s)
+          for r, s in ((12, 16), (32, 0))]
     c.append(dict(megakernel=1))
     return c
 
