@@ -539,25 +539,13 @@ __global__ void __launch_bounds__(SORT_THREADS) k_sort_small(u64* __restrict__ k
 		const int shift = 8 * pass;
 		for(int i = tid; i < SORT_WARPS * 256; i += SORT_THREADS) sWarpHist[i] = 0;
 		__syncthreads();
+		unsigned peers[SORT_ITEMS];
 #pragma unroll
-		for(int i = 0; i < SORT_ITEMS; ++i) {
-			const bool valid = base + uint32_t(i) * 32 + lane < n;
-			const uint32_t d = uint32_t(k[i] >> shift) & 255u;
-			const unsigned vm = __ballot_sync(0xffffffffu, valid);
-			rank[i] = 0;
-			if(valid) {
-				const unsigned peers = __match_any_sync(vm, d);
-				const int leader = __ffs(peers) - 1;
-				uint32_t prev = 0;
-				if(int(lane) == leader) {
-					prev = sWarpHist[warp * 256 + d];
-					sWarpHist[warp * 256 + d] = prev + __popc(peers);
-				}
-				prev = __shfl_sync(peers, prev, leader);
-				rank[i] = prev + __popc(peers & lt);
-			}
-			__syncwarp();
-		}
+		for(int i = 0; i < SORT_ITEMS; ++i)
+			peers[i] = digit_peers(uint32_t(k[i] >> shift) & 255u, base + uint32_t(i) * 32 + lane < n);
+#pragma unroll
+		for(int i = 0; i < SORT_ITEMS; ++i)
+			rank[i] = digit_rank(sWarpHist + warp * 256, uint32_t(k[i] >> shift) & 255u, peers[i], lane, lt);
 		__syncthreads();
 		// thread d: digit d's count per warp made exclusive, then its place in the block
 		uint32_t total = 0;
@@ -567,16 +555,7 @@ __global__ void __launch_bounds__(SORT_THREADS) k_sort_small(u64* __restrict__ k
 			sWarpHist[w * 256 + tid] = total;
 			total += c;
 		}
-		uint32_t incl = total;
-		for(int off = 1; off < 32; off <<= 1) {
-			const uint32_t x = __shfl_up_sync(0xffffffffu, incl, off);
-			if(lane >= unsigned(off)) incl += x;
-		}
-		if(lane == 31u) sWarpSum[warp] = incl;
-		__syncthreads();
-		uint32_t before = 0;
-		for(int w = 0; w < warp; ++w) before += sWarpSum[w];
-		sStart[tid] = before + incl - total;
+		sStart[tid] = digit_start(total, sWarpSum, lane, warp);
 		__syncthreads();
 #pragma unroll
 		for(int i = 0; i < SORT_ITEMS; ++i) {

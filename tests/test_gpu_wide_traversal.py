@@ -96,3 +96,15 @@ def test_short_sorts_are_stable(dll, n, distinct):
     gk, gv = bindings.sort_pairs(dll, k, v)
     order = np.argsort(k, kind="stable")
     assert np.array_equal(gk, k[order]) and np.array_equal(gv, v[order])
+
+
+# tiles of 2 048 pairs: full ones, one pair over and one short; digits that all lanes of a warp share, and random ones
+@pytest.mark.parametrize("distinct", [2, 1 << 60])
+@pytest.mark.parametrize("n", [9 * 2048, 9 * 2048 + 1, 17 * 2048 - 1, 130 * 2048 + 31])
+def test_tiled_sorts_are_stable(dll, n, distinct):
+    rng = np.random.default_rng(n)
+    k = np.sort(rng.integers(0, distinct, n, dtype=np.uint64)) if distinct == 2 else rng.integers(0, distinct, n, dtype=np.uint64)
+    v = np.arange(n, dtype=np.int32)
+    gk, gv = bindings.sort_pairs(dll, k, v)
+    order = np.argsort(k, kind="stable")
+    assert np.array_equal(gk, k[order]) and np.array_equal(gv, v[order])
