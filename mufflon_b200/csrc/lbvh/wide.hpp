@@ -13,9 +13,10 @@
 //   * 80-byte node, five 16-byte loads;
 //   * every quantised box contains its child's exact box with a margin of one
 //     grid step on every side (directed rounding), so that the box test,
-//     computed as t = q * (2^e * invDir) + (p - origin) * invDir, never culls a
+//     t = (q + 2^15) * (2^e * invDir) + ((p - origin) * invDir - 2^15 * 2^e * invDir)
+//     with the second term rounded outwards (wide_traverse.cuh), never culls a
 //     box that contains a hit point (the step is far larger than the rounding
-//     error of that expression);
+//     error of the rest);
 //   * leaves hold at most wide_leaf_max primitives of one contiguous range;
 //     meta[slot] = (one bit per primitive << 5) | offset, offset relative to
 //     the node's primitive base, and (1 << 5) | (24 + slot) for an internal

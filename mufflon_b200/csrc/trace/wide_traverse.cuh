@@ -145,10 +145,15 @@ MBD float max3_(float a, float b, float c) {
 // With a plane's byte read as q + 2^15, its distance is one multiply-add:
 //   (q + 2^15) * s + (o - 2^15 * s),
 // near and far plane of an axis in one packed instruction. The additive
-// constant is rounded to 2^-9 of a grid step, and the far-plane tolerance is
-// applied to the per-node scale and offset, not per child: both move a plane
-// by far less than the grid step of margin every quantised box carries, so
-// the test stays conservative.
+// constants are rounded outwards, the near plane's down and the far plane's up,
+// so their rounding (at most 2^-8 of a grid step, or 2^-23 of the offset if that
+// is larger) only widens a box. That holds
+// at any scale: where 2^15 * s overflows (grid steps from 2^49 on, and a ray
+// along a coordinate axis), the near constant becomes -inf or stays the largest
+// finite number, the far one +inf or stays the smallest, and the box is kept.
+// The far-plane tolerance is applied to the per-node scale and offset, not per
+// child, which moves a plane by far less than the grid step of margin every
+// quantised box carries.
 MBD void wide_node_test(const WideNode* nodes, uint32_t idx, f3 org, f3 inv, uint32_t oct, float tmaxBox,
                         uint32_t& ngBase, uint32_t& ngMask, uint32_t& pgBase, uint32_t& pgHits) {
 	const float4* q = reinterpret_cast<const float4*>(nodes + idx);
@@ -159,7 +164,7 @@ MBD void wide_node_test(const WideNode* nodes, uint32_t idx, f3 org, f3 inv, uin
 		const float t = __fmul_rn(__fsub_rn(grid, o), i);
 		const float fs = __fmul_rn(s, BOX_FAR_SLACK), ft = __fmul_rn(t, BOX_FAR_SLACK);
 		s2 = pack2(s, fs);
-		o2 = pack2(__fmaf_rn(-QBYTE_BIAS, s, t), __fmaf_rn(-QBYTE_BIAS, fs, ft));
+		o2 = pack2(__fmaf_rd(-QBYTE_BIAS, s, t), __fmaf_ru(-QBYTE_BIAS, fs, ft));
 	};
 	unsigned long long sx, sy, sz, ox, oy, oz;
 	axis(n0.x, eim & 0xFFu, org.x, inv.x, sx, ox);

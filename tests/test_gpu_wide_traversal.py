@@ -86,6 +86,39 @@ def test_hits_and_occlusion_bit_exact(dll, oracle, n, instances, offset):
     assert np.array_equal(dll.trace_occlusion(a, b), sc.trace_any(a, b))
 
 
+# Coordinates up to 2^58: the box test's products with a clamped reciprocal direction reach the end of the 32-bit
+# range (2^49 grid steps of 2^15 at a reciprocal of 2^64, and above), for the object's level and the instances'.
+@pytest.mark.parametrize("exponent", [0, 40, 54, 56, 58])
+@pytest.mark.parametrize("instances", [1, 3])
+def test_axis_rays_at_any_scale(dll, oracle, exponent, instances):
+    size = 2.0 ** exponent
+    rng = np.random.default_rng(exponent)
+    n = 60
+    sph = np.concatenate([rng.uniform(-1.0, 1.0, (n, 3)), rng.uniform(0.05, 0.2, (n, 1))], 1) * size
+    lod = scenes.LodSpec(np.zeros((0, 3), np.float32), np.zeros((0, 3), np.float32), np.zeros((0, 2), np.float32),
+                         np.zeros((0, 3), np.uint32), np.zeros((0, 4), np.uint32), np.zeros(0, np.uint16),
+                         sph.astype(np.float32), np.zeros(n, np.uint16), name="spheres")
+    spec = _spec(1, instances, np.zeros(3), 1)
+    spec.lods[0] = lod
+    spec.world_to_instance = np.tile(np.array(scenes.identity34(), np.float32), (instances, 1))
+    spec.world_to_instance[:, 3] = np.arange(instances) * np.float32(0.7 * size)
+    dll.world_clear_all()
+    bindings.load_scene_spec(dll, spec)
+    assert dll.render_enable_renderer(0, 0)
+    assert dll.renderer_set_parameter_int("Megakernel", 0)
+    sc = oracle.OracleScene(spec)
+    m = 3000
+    d = np.where(rng.uniform(size=(m, 3)) < 0.5, 0.0, -0.0)
+    d[np.arange(m), rng.integers(0, 3, m)] = np.where(rng.uniform(size=m) < 0.5, -1.0, 1.0)
+    rays = np.concatenate([rng.uniform(-1.2, 1.2, (m, 3)) * size, d], 1).astype(np.float32)
+    tmax = float(8.0 * size)
+    gt, gi, gp, gs = dll.trace_rays(rays, tmax=tmax)
+    ot, oi, op, _ = sc.trace_first(rays, tmax=tmax)
+    assert (oi >= 0).sum() > m // 10
+    assert np.array_equal(gi, oi) and np.array_equal(gp, op)
+    assert np.array_equal(gt.view(np.uint32), ot.view(np.uint32))
+
+
 # either side of the single-block sort's capacity, few distinct keys and many
 @pytest.mark.parametrize("distinct", [3, 1 << 60])
 @pytest.mark.parametrize("n", [31, 257, 2047, 2048, 2049])
