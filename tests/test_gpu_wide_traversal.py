@@ -3,11 +3,13 @@ no hierarchy (one primitive), a root of leaves only, full leaves, the first root
 one instance (entered without an instance level) or several; boxes far from the rays' origins, where the
 box test's rounding is largest against its one-grid-step margin."""
 import math
+import os
+import subprocess
 
 import numpy as np
 import pytest
 
-from mufflon_b200 import bindings, scenes
+from mufflon_b200 import bindings, build, scenes
 
 pytestmark = pytest.mark.gpu
 
@@ -117,6 +119,18 @@ def test_axis_rays_at_any_scale(dll, oracle, exponent, instances):
     assert (oi >= 0).sum() > m // 10
     assert np.array_equal(gi, oi) and np.array_equal(gp, op)
     assert np.array_equal(gt.view(np.uint32), ot.view(np.uint32))
+
+
+def test_box_reciprocal_is_correctly_rounded(tmp_path):
+    """Every float of these exponents, zeros and denormals among them: the bits of the IEEE reciprocal."""
+    exe = str(tmp_path / "box_reciprocal")
+    source = os.path.join(build.ROOT, "tests", "cpp", "box_reciprocal.cu")
+    flags = [f for f in build.NVCC_FLAGS if f not in ("-Xptxas", "-v")]
+    subprocess.run([build.NVCC, *flags, source, "-o", exe], check=True, capture_output=True)
+    exponents = [-127, -126, -97, -65, -64, -63, -37, -17, -7, -2, -1, 0, 1, 13, 63, 125]
+    r = subprocess.run([exe, *map(str, exponents)], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0
+    assert [int(x) for x in r.stdout.split()] == [0] * len(exponents)
 
 
 # either side of the single-block sort's capacity, few distinct keys and many
