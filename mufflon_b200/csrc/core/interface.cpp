@@ -1472,29 +1472,15 @@ Boolean render_iterate(MufflonInstanceHdl h, ProcessTime* iterTime, ProcessTime*
 	CHECK_CUDA(cudaEventRecord(r.evStop, I.stream));
 	const TraceCounters* both = r.link->counters;
 	CHECK_CUDA(cudaMemcpyAsync(r.link->counters, r.counters, 2 * sizeof(TraceCounters), cudaMemcpyDeviceToHost, I.stream));
-	const unsigned* bounceQueue = r.link->bounceQueue;
 	if(!r.megakernel)
 		CHECK_CUDA(cudaMemcpyAsync(r.link->bounceQueue, r.wf.counters + WF_COUNTERS - WF_BOUNCE_STATS,
 		                           sizeof(r.link->bounceQueue), cudaMemcpyDeviceToHost, I.stream));
 	CHECK_CUDA(cudaStreamSynchronize(I.stream));
 	if(!r.megakernel) {
-		// next iteration's plan: the first bounce >= wavefrontBounces whose
-		// extension queue held at most tailPaths paths and whose remaining
-		// vertices cost less in the tail launch than in launches of their own
-		// (none: no tail). A plan stays while it is near that line, so that the
-		// captured graph is not made again for a queue that varies about it.
-		const int maxB = std::max(1, r.params.maxPathLength);
-		const bool same = planKey == r.planKey;
-		int plan = maxB;
-		for(int b = std::max(0, r.wavefrontBounces); b + 1 < maxB && b < int(WF_BOUNCE_STATS); ++b) {
-			if(bounceQueue[b] <= unsigned(std::max(0, r.tailPaths)) &&
-			   tail_pays(bounceQueue[b], b > 0 ? bounceQueue[b - 1] : 0u, maxB - 1 - b, std::max(1, r.params.neeCount),
-			             same && r.plannedTail == b ? 1.5f : 1.0f)) {
-				plan = b;
-				break;
-			}
-		}
-		r.plannedTail = plan;
+		// next iteration's plan
+		const int keep = planKey == r.planKey ? r.plannedTail : -1;
+		r.plannedTail = plan_tail(r.link->bounceQueue, std::max(1, r.params.maxPathLength), r.wavefrontBounces, r.tailPaths,
+		                          std::max(1, r.params.neeCount), tune.tailBounce, keep);
 		r.planKey = planKey;
 	}
 	CHECK_CUDA(cudaEventElapsedTime(&r.lastKernelMs, r.evStart, r.evStop));

@@ -77,6 +77,25 @@ inline bool tail_pays(unsigned paths, unsigned before, int bounces, int neeCount
 	return rays * (TAIL_NS + TAIL_LONG_NS * further) <= slack * (rays * WAVE_NS + launches * BOUNCE_NS);
 }
 
+// The bounce at which the next iteration's tail launch takes over, from the
+// queue length of each bounce of this one (WF_BOUNCE_STATS entries): the first
+// bounce >= firstBounce with at most tailPaths paths that tail_pays();
+// maxBounces: none; -1: to be decided on the device. `launched` is this
+// iteration's own hand-over (-1: decided on the device): no queue length was
+// recorded after it, so if none of the bounces up to it qualifies, the next
+// iteration is left to the device, which sees every length. `keep` is a plan that stays
+// while it is near the line (-1: none), so that the captured graph is not made
+// again for a queue that varies about it.
+inline int plan_tail(const unsigned* queue, int maxBounces, int firstBounce, int tailPaths, int neeCount, int launched, int keep) {
+	const unsigned most = tailPaths > 0 ? unsigned(tailPaths) : 0u;
+	for(int b = firstBounce > 0 ? firstBounce : 0; b + 1 < maxBounces && b < int(WF_BOUNCE_STATS); ++b) {
+		if(launched >= 0 && b > launched) return -1;
+		if(queue[b] <= most && tail_pays(queue[b], b > 0 ? queue[b - 1] : 0u, maxBounces - 1 - b, neeCount, keep == b ? 1.5f : 1.0f))
+			return b;
+	}
+	return maxBounces;
+}
+
 // WF_EXTEND: the trace launches of the wavefront bounces (extension and
 // shadow rays); WF_TAIL: the launch that finishes the remaining paths.
 // WF_BIN: the scan and scatter launches that order queued rays by coherence.
