@@ -8,7 +8,9 @@ parameters and keeps the fastest:
 * "Trace blocks per SM": the trace kernel's register budget (block shape);
 * "Wavefront bounces" and "Tail paths": how many bounces always run as
   separate launches, and the queue length at or below which one launch
-  finishes the remaining paths;
+  may finish the remaining paths;
+* "Tail cost rule": whether it does so only where the estimate of its cost
+  says that it pays;
 * "Trace refill lanes": how many idle lanes of a warp are refilled together;
 * "Ray sort bits": the resolution of the coherence binning of queued rays
   (0: traced in queue order).
@@ -25,12 +27,14 @@ from typing import Dict, List, Optional
 
 PARAMS = {"megakernel": "Megakernel", "trace_blocks": "Trace blocks per SM",
           "wavefront_bounces": "Wavefront bounces", "refill_lanes": "Trace refill lanes", "tail_paths": "Tail paths",
-          "sort_bits": "Ray sort bits"}
+          "tail_cost": "Tail cost rule", "sort_bits": "Ray sort bits"}
 
 
 def default_candidates() -> List[Dict[str, int]]:
-    c = [dict(megakernel=0, trace_blocks=b, wavefront_bounces=k, refill_lanes=12, tail_paths=t)
-         for b, k, t in itertools.product((4, 6), (1, 2), (32768, 98304, 262144))]
+    c = [dict(megakernel=0, trace_blocks=b, wavefront_bounces=2, refill_lanes=12, tail_paths=98304, tail_cost=1)
+         for b in (4, 6)]
+    c += [dict(megakernel=0, trace_blocks=b, wavefront_bounces=k, refill_lanes=12, tail_paths=t, tail_cost=0)
+          for b, k, t in itertools.product((4, 6), (1, 2), (32768, 262144))]
     c += [dict(megakernel=0, trace_blocks=6, wavefront_bounces=2, refill_lanes=r, tail_paths=98304, sort_bits=s)
           for r, s in ((12, 16), (32, 0))]
     c.append(dict(megakernel=1))

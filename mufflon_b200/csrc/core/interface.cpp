@@ -61,7 +61,7 @@ const ParamDesc PT_PARAMS[] = {
 	{ "Stage timing", PARAM_INT }, { "Traversal statistics", PARAM_INT }, { "Trace blocks per SM", PARAM_INT }, { "Wavefront bounces", PARAM_INT },
 	{ "Trace refill lanes", PARAM_INT }, { "Tail paths", PARAM_INT }, { "Iteration graph", PARAM_INT },
 	{ "Planned tail", PARAM_INT }, { "Ray sort bits", PARAM_INT }, { "Ray sort direction bits", PARAM_INT },
-	{ "Traversal step limit", PARAM_INT },
+	{ "Traversal step limit", PARAM_INT }, { "Tail cost rule", PARAM_INT },
 };
 // lt_params.hpp:8-12, plus the recording switch of the parity tests
 const ParamDesc LT_PARAMS[] = {
@@ -116,6 +116,7 @@ int32_t* param_ptr(RendererState& r, const char* name) {
 	if(!std::strcmp(name, "Tail paths")) return &r.tailPaths;
 	if(!std::strcmp(name, "Iteration graph")) return &r.iterationGraph;
 	if(!std::strcmp(name, "Planned tail")) return &r.planTail;
+	if(!std::strcmp(name, "Tail cost rule")) return &r.tailCost;
 	if(!std::strcmp(name, "Ray sort bits")) return &r.sortBits;
 	if(!std::strcmp(name, "Ray sort direction bits")) return &r.sortDirBits;
 	return nullptr;
@@ -1415,6 +1416,7 @@ Boolean render_iterate(MufflonInstanceHdl h, ProcessTime* iterTime, ProcessTime*
 	tune.wavefrontBounces = r.wavefrontBounces;
 	tune.refillLanes = r.refillLanes;
 	tune.tailPaths = r.tailPaths;
+	tune.tailCost = r.tailCost;
 	tune.sortBits = r.sortBits;
 	tune.sortDirBits = r.sortDirBits;
 	tune.counters = r.traversalStats != 0; // the counting kernel variants only when asked for
@@ -1425,7 +1427,7 @@ Boolean render_iterate(MufflonInstanceHdl h, ProcessTime* iterTime, ProcessTime*
 	{
 		auto addp = [&](const void* p, size_t b) { const unsigned char* c = static_cast<const unsigned char*>(p); planKey.insert(planKey.end(), c, c + b); };
 		addp(&I.scene.desc, sizeof(DScene)); addp(&r.params, sizeof(PtParams));
-		addp(&r.wavefrontBounces, sizeof(int32_t)); addp(&r.tailPaths, sizeof(int32_t));
+		addp(&r.wavefrontBounces, sizeof(int32_t)); addp(&r.tailPaths, sizeof(int32_t)); addp(&r.tailCost, sizeof(int32_t));
 		addp(&r.width, sizeof(r.width)); addp(&r.height, sizeof(r.height));
 	}
 	if(!r.megakernel && r.planTail && planKey == r.planKey) tune.tailBounce = r.plannedTail;
@@ -1480,7 +1482,7 @@ Boolean render_iterate(MufflonInstanceHdl h, ProcessTime* iterTime, ProcessTime*
 		// next iteration's plan
 		const int keep = planKey == r.planKey ? r.plannedTail : -1;
 		r.plannedTail = plan_tail(r.link->bounceQueue, std::max(1, r.params.maxPathLength), r.wavefrontBounces, r.tailPaths,
-		                          std::max(1, r.params.neeCount), tune.tailBounce, keep);
+		                          std::max(1, r.params.neeCount), tune.tailCost != 0, tune.tailBounce, keep);
 		r.planKey = planKey;
 	}
 	CHECK_CUDA(cudaEventElapsedTime(&r.lastKernelMs, r.evStart, r.evStop));
@@ -1883,6 +1885,7 @@ Boolean mufflon_render_batch(const MufflonBatchJob* jobs, uint32_t count, int32_
 	tune.wavefrontBounces = r0.wavefrontBounces;
 	tune.refillLanes = r0.refillLanes;
 	tune.tailPaths = r0.tailPaths;
+	tune.tailCost = r0.tailCost;
 	tune.sortBits = r0.sortBits;
 	tune.sortDirBits = r0.sortDirBits;
 	tune.counters = false;
@@ -2038,6 +2041,7 @@ static void run_adjoint(MufflonInstance& I, uint32_t spp, const float* imageGrad
 		tune.wavefrontBounces = r.wavefrontBounces;
 		tune.refillLanes = r.refillLanes;
 		tune.tailPaths = r.tailPaths;
+		tune.tailCost = r.tailCost;
 		tune.sortBits = r.sortBits;
 		tune.sortDirBits = r.sortDirBits;
 		tune.counters = false;

@@ -215,6 +215,7 @@ struct RendererState {
 	int32_t wavefrontBounces = 2; // bounces run as separate stage launches before the tail launch
 	int32_t refillLanes = 12;     // idle trace lanes refilled together
 	int32_t tailPaths = 98304;    // queue length at or below which the tail launch takes over
+	int32_t tailCost = 1;         // "Tail cost rule": ... and only if it pays (tail_pays)
 	int32_t iterationGraph = 1;   // replay the wavefront launches of an iteration as one CUDA graph
 	int32_t planTail = 1;         // plan the tail bounce from the previous iteration's queue lengths
 	int32_t stepLimit = 0;        // "Traversal step limit" of every renderer; 0: MAX_TRAVERSAL_STEPS

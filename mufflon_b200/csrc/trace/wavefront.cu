@@ -721,7 +721,8 @@ MBD void shade_slot(const SP& sp, WfState& W, int q, int bounce, unsigned slot) 
 
 // Whether the tail launch takes the `count` paths of `bounce`, decided alike
 // by the tail and the shade launch of an unplanned iteration; tailBounces: the
-// bounces that may follow, negative where the tail may not take over.
+// bounces that may follow, negative where the tail may not take over, 0 where
+// it does so whatever it costs.
 MBD bool tail_takes(const WfState& W, unsigned count, int bounce, int neeCount, unsigned tailMax, int tailBounces) {
 	if(tailBounces < 0 || count > tailMax) return false;
 	// the trace launches record every bounce's queue length
@@ -1275,7 +1276,7 @@ void run_bounces(const SP& sp, WfState W, TraceCounters* counters, uint32_t numP
 		// From bounce wavefrontBounces on, the first bounce whose queue holds
 		// at most tailMax paths, and pays, is finished by one launch (decided on the
 		// device from the queue length); the later launches return at once.
-		const int tailBounces = b >= tuning.wavefrontBounces && b + 1 < maxBounces ? maxBounces - 1 - b : -1;
+		const int tailBounces = b >= tuning.wavefrontBounces && b + 1 < maxBounces ? (tuning.tailCost ? maxBounces - 1 - b : 0) : -1;
 		if(tailBounces >= 0) {
 			const TailKernel<SP> tl = tail_kernel<SP>(tuning.counters, tuning.alpha);
 			log.begin(WF_TAIL);

@@ -54,7 +54,7 @@ constexpr unsigned WF_BOUNCE_STATS = 64;
 
 // Whether the tail launch should finish a queue of `paths` paths, left of the
 // previous bounce's `before` (0: unknown), with up to `bounces` bounces to
-// come. The tail runs a path's vertices one after the other with few lanes
+// come (0: it always should, the renderer parameter "Tail cost rule" is off). The tail runs a path's vertices one after the other with few lanes
 // per instruction, and worse the longer its paths are; launches of their own
 // cost more per bounce than per vertex. The line was fitted to these times of
 // what remains after two bounces, tail against launches (ms per iteration;
@@ -86,11 +86,13 @@ inline bool tail_pays(unsigned paths, unsigned before, int bounces, int neeCount
 // iteration is left to the device, which sees every length. `keep` is a plan that stays
 // while it is near the line (-1: none), so that the captured graph is not made
 // again for a queue that varies about it.
-inline int plan_tail(const unsigned* queue, int maxBounces, int firstBounce, int tailPaths, int neeCount, int launched, int keep) {
+inline int plan_tail(const unsigned* queue, int maxBounces, int firstBounce, int tailPaths, int neeCount, bool costRule,
+                     int launched, int keep) {
 	const unsigned most = tailPaths > 0 ? unsigned(tailPaths) : 0u;
 	for(int b = firstBounce > 0 ? firstBounce : 0; b + 1 < maxBounces && b < int(WF_BOUNCE_STATS); ++b) {
 		if(launched >= 0 && b > launched) return -1;
-		if(queue[b] <= most && tail_pays(queue[b], b > 0 ? queue[b - 1] : 0u, maxBounces - 1 - b, neeCount, keep == b ? 1.5f : 1.0f))
+		if(queue[b] <= most && tail_pays(queue[b], b > 0 ? queue[b - 1] : 0u, costRule ? maxBounces - 1 - b : 0, neeCount,
+		                                 keep == b ? 1.5f : 1.0f))
 			return b;
 	}
 	return maxBounces;
@@ -122,6 +124,7 @@ struct WfTuning {
 	                           // that tail_pays() is finished by one launch that runs every remaining
 	                           // path in place
 	int tailPaths = 98304;
+	int tailCost = 1;          // 0: at the first such bounce whether or not it pays
 	int tailBounce = -1;       // >= 0: planned schedule, the tail launch takes over at this bounce and
 	                           // nothing is launched after it; -1: decided on the device per bounce
 	int refillLanes = 12;      // idle lanes of a trace warp are refilled together once this many are idle (1..32)

@@ -133,7 +133,8 @@ def test_lbvh_bit_exact_full_icosphere(dll, oracle):
 # kernel over the binary (reference-layout) hierarchies.
 KERNELS = {"wavefront": 0, "megakernel": 1}
 DEFAULT_PARAMS = {"Seed": 0, "Min. path length": 0, "Max. path length": 16, "NEE count": 1,
-                  "RR start depth": 0, "Megakernel": 0, "Wavefront bounces": 2, "Tail paths": 98304, "Iteration graph": 1,
+                  "RR start depth": 0, "Megakernel": 0, "Wavefront bounces": 2, "Tail paths": 98304, "Tail cost rule": 1,
+                  "Iteration graph": 1,
                   "Planned tail": 1, "Ray sort bits": 12, "Ray sort direction bits": 3}
 
 
@@ -327,18 +328,22 @@ def test_pt_multi_nee_min_path_parity(dll, oracle, kernel):
                                                            (1, 0), (1, 2500)])
 def test_pt_schedule_parity(dll, oracle, wavefront_bounces, tail_paths):
     """Any split between per-bounce stage launches and the path-finishing launch gives the oracle's bits
-    (tail_paths 2500 hands over in the middle of the paths, 0 never before the queues are empty)."""
+    (whatever the hand-over costs: tail_paths 98304 at wavefront_bounces, 2500 in the middle of the paths, 0 never
+    before the queues are empty)."""
     spec = scenes.cornell_box(5, 80, 80)
     _load(dll, spec)
     dll.render_enable_render_target("Radiance", False)
     dll.render_enable_render_target("Hit ID", False)
-    for name, value in {"Wavefront bounces": wavefront_bounces, "Tail paths": tail_paths, "NEE count": 2,
+    for name, value in {"Wavefront bounces": wavefront_bounces, "Tail paths": tail_paths, "Tail cost rule": 0, "NEE count": 2,
                         "Max. path length": 9, "RR start depth": 2, "Min. path length": 1}.items():
         assert dll.renderer_set_parameter_int(name, value)
     pt = oracle.OraclePathTracer(oracle.OracleScene(spec), seed=0, min_path=1, max_path=9, nee_count=2, rr_start=2)
     for _ in range(2):
         dll.render_iterate()
         pt.iterate()
+    # the planned second iteration: trace, shade, scan and scatter for each bounce before the hand-over, then one launch
+    if tail_paths == 98304 and wavefront_bounces < 8:
+        assert dll.stage_stats()["launches"] == 4 + 4 * wavefront_bounces
     assert np.array_equal(dll.get_target_image("Hit ID"), pt.target("Hit ID"))
     assert rel_rmse(dll.get_target_image("Radiance"), pt.target("Radiance")) <= RMSE_TOL
 

@@ -14,9 +14,9 @@ def plan(tmp_path_factory):
     subprocess.run(["g++", "-std=c++17", "-ffp-contract=off", f"-I{cuda}/include", os.path.join(ROOT, "tests", "cpp", "tail_plan.cpp"),
                     "-o", exe], check=True, capture_output=True)
 
-    def run(queues, max_bounces=8, first=2, tail_paths=98304, nee=1, launched=-1, keep=-1):
+    def run(queues, max_bounces=8, first=2, tail_paths=98304, nee=1, cost=1, launched=-1, keep=-1):
         many = isinstance(queues[0], list)
-        lines = [" ".join(str(x) for x in (max_bounces, first, tail_paths, nee, launched, keep, len(q), *q))
+        lines = [" ".join(str(x) for x in (max_bounces, first, tail_paths, nee, cost, launched, keep, len(q), *q))
                  for q in (queues if many else [queues])]
         out = subprocess.run([exe], input="\n".join(lines), check=True, capture_output=True, text=True).stdout.split()
         return [int(x) for x in out] if many else int(out[0])
@@ -56,3 +56,10 @@ def test_a_plan_stays_near_the_line(plan):
     at = 1 + plan([[10 * q, 2 * q, q] for q in range(1, 98304)], launched=2).index(-1)
     assert plan([10 * at, 2 * at, at], launched=2, keep=2) == 2
     assert plan([10 * at, 2 * at, at], launched=2, keep=1) == -1
+
+
+def test_without_the_cost_rule_only_the_length_counts(plan):
+    assert plan(LONG, cost=0, tail_paths=800_000) == 2
+    assert plan(LONG, cost=0, tail_paths=600_000) == 4
+    assert plan(LONG, cost=0, first=0, tail_paths=1 << 30) == 0
+    assert plan(LONG[:4], cost=0, tail_paths=98304, launched=3) == -1
