@@ -35,7 +35,7 @@ LOADER_SOURCES = ["loader/json.cpp", "loader/mff_binary.cpp", "loader/scene_load
 LOADER_HEADERS = ["loader/json.hpp", "loader/mff_binary.hpp", "loader/scene_loader.hpp"]
 HEADERS = ["common/fmath.hpp", "common/pfm.hpp", "trace/dmath.cuh", "trace/intersect.cuh", "trace/shading.cuh",
            "trace/scene_types.hpp", "trace/pt_api.hpp", "lbvh/lbvh.hpp", "lbvh/radix_sort.cuh",
-           "lbvh/sort_noalloc.hpp", "trace/wavefront.hpp", "trace/wide_traverse.cuh", "lbvh/wide.hpp", "core/world.hpp",
+           "lbvh/sort_noalloc.hpp", "trace/wavefront.hpp", "trace/wide_traverse.cuh", "lbvh/wide.hpp", "core/world.hpp", "core/call_scratch.hpp",
            "core/light_build.hpp", "core/instance_boxes.hpp", "trace/lt_api.hpp",
            "trace/emit.cuh", "trace/accumulate.cuh", "trace/ray_queue.cuh", "trace/bidir.cuh", "trace/aux_targets.cuh"]
 

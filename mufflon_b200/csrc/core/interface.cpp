@@ -431,20 +431,6 @@ void RendererState::release() {
 	evStart = evStop = nullptr;
 	width = height = 0;
 }
-cudaError_t CallScratch::reserve(size_t need) {
-	if(need <= bytes) return cudaSuccess;
-	release();
-	const cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&device), need);
-	if(e != cudaSuccess) { device = nullptr; return e; }
-	bytes = need;
-	return cudaSuccess;
-}
-void CallScratch::trim() { if(bytes > KEEP) release(); }
-void CallScratch::release() {
-	cudaFree(device);
-	device = nullptr;
-	bytes = 0;
-}
 MufflonInstance::~MufflonInstance() {
 	renderer.release();
 	scratch.release();
@@ -2005,13 +1991,14 @@ static void run_adjoint(MufflonInstance& I, uint32_t spp, const float* imageGrad
 		ensure_wavefront_buffers(I);
 	}
 	try {
+		CallScratchUse scratch(I.scratch, I.stream);
 		// one slab of the kept scratch memory: the replay's bookkeeping,
 		// generators, image gradient, texel gradient, emission gradient and flags
 		const size_t adjBytes = wavefront ? align256(adjoint_bytes(n, r.params.maxPathLength)) : 0;
 		const size_t gradBytes = texIndex >= 0 ? align256(nt * 12) : 0;
 		const size_t flagBytes = emitTarget ? align256(emitTarget->size()) : 0;
-		CHECK_CUDA(I.scratch.reserve(adjBytes + align256(n * 8) + align256(n * 12) + gradBytes + 256 + flagBytes));
-		char* m = I.scratch.device;
+		CHECK_CUDA(scratch.reserve(adjBytes + align256(n * 8) + align256(n * 12) + gradBytes + 256 + flagBytes));
+		char* m = scratch.data();
 		auto take = [&](size_t bytes) { char* p = m; m += bytes; return p; };
 		void* adjMem = take(adjBytes);
 		uint64_t* rng = reinterpret_cast<uint64_t*>(take(align256(n * 8)));
@@ -2058,8 +2045,7 @@ static void run_adjoint(MufflonInstance& I, uint32_t spp, const float* imageGrad
 		if(emitTarget) CHECK_CUDA(cudaMemcpyAsync(emisGradOut, dEmis, 12, cudaMemcpyDeviceToHost, I.stream));
 		TraceCounters tc[2] = {};
 		if(wavefront) CHECK_CUDA(cudaMemcpyAsync(tc, r.counters, sizeof(tc), cudaMemcpyDeviceToHost, I.stream));
-		CHECK_CUDA(cudaStreamSynchronize(I.stream));
-		I.scratch.trim();
+		CHECK_CUDA(scratch.finish());
 		if(deviceMs) CHECK_CUDA(cudaEventElapsedTime(deviceMs, a, b));
 		check_traversal(tc[0].errors + tc[1].errors, desc.maxSteps);
 	} catch(...) {
@@ -2175,8 +2161,9 @@ Boolean mufflon_trace_rays(MufflonInstanceHdl h, const float* rays, const float*
 	if(n == 0) return true;
 	const size_t N = n;
 	auto part = [](size_t bytes) { return align256(bytes); };
-	CHECK_CUDA(I.scratch.reserve(part(N * 24) + 3 * part(N * 4) + part(N * 8) + (geo ? N * 12 : 0)));
-	char* m = I.scratch.device;
+	CallScratchUse scratch(I.scratch, I.stream);
+	CHECK_CUDA(scratch.reserve(part(N * 24) + 3 * part(N * 4) + part(N * 8) + (geo ? N * 12 : 0)));
+	char* m = scratch.data();
 	auto take = [&](size_t bytes) { char* p = m; m += part(bytes); return p; };
 	float* dr = reinterpret_cast<float*>(take(N * 24));
 	float* dt = reinterpret_cast<float*>(take(N * 4));
@@ -2192,8 +2179,7 @@ Boolean mufflon_trace_rays(MufflonInstanceHdl h, const float* rays, const float*
 	CHECK_CUDA(cudaMemcpyAsync(inst, di, N * 4, cudaMemcpyDeviceToHost, I.stream));
 	CHECK_CUDA(cudaMemcpyAsync(prim, dp, N * 4, cudaMemcpyDeviceToHost, I.stream));
 	if(sp) CHECK_CUDA(cudaMemcpyAsync(sp, dsp, N * 8, cudaMemcpyDeviceToHost, I.stream));
-	CHECK_CUDA(cudaStreamSynchronize(I.stream));
-	I.scratch.trim();
+	CHECK_CUDA(scratch.finish());
 	return true;
 	CATCH_ALL(false)
 }
@@ -2206,17 +2192,17 @@ Boolean mufflon_trace_occlusion(MufflonInstanceHdl h, const float* a, const floa
 	load_scene_if_needed(I);
 	if(n == 0) return true;
 	const size_t points = align256(size_t(n) * 12);
-	CHECK_CUDA(I.scratch.reserve(2 * points + n));
-	float* da = reinterpret_cast<float*>(I.scratch.device);
-	float* db = reinterpret_cast<float*>(I.scratch.device + points);
-	uint8_t* dout = reinterpret_cast<uint8_t*>(I.scratch.device + 2 * points);
+	CallScratchUse scratch(I.scratch, I.stream);
+	CHECK_CUDA(scratch.reserve(2 * points + n));
+	float* da = reinterpret_cast<float*>(scratch.data());
+	float* db = reinterpret_cast<float*>(scratch.data() + points);
+	uint8_t* dout = reinterpret_cast<uint8_t*>(scratch.data() + 2 * points);
 	CHECK_CUDA(cudaMemcpyAsync(da, a, size_t(n) * 12, cudaMemcpyHostToDevice, I.stream));
 	CHECK_CUDA(cudaMemcpyAsync(db, b, size_t(n) * 12, cudaMemcpyHostToDevice, I.stream));
 	if(I.renderer.megakernel) CHECK_CUDA(launch_occlusion(I.scene.desc, da, db, n, dout, I.stream));
 	else CHECK_CUDA(launch_occlusion_wide(I.scene.desc, da, db, n, dout, I.stream));
 	CHECK_CUDA(cudaMemcpyAsync(occ, dout, n, cudaMemcpyDeviceToHost, I.stream));
-	CHECK_CUDA(cudaStreamSynchronize(I.stream));
-	I.scratch.trim();
+	CHECK_CUDA(scratch.finish());
 	return true;
 	CATCH_ALL(false)
 }

@@ -16,6 +16,7 @@
 
 #include <cuda_runtime.h>
 
+#include "call_scratch.hpp"
 #include "../../../include/mufflon_core.h"
 #include "../trace/scene_types.hpp"
 #include "../lbvh/lbvh.hpp"
@@ -301,21 +302,6 @@ struct RendererState {
 	float* screen = nullptr;       // page-locked copy of the last target read back (library-owned)
 	size_t screenCap = 0;          // its capacity in floats
 	int screenChannels = 0;
-	void release();
-};
-
-// Device memory that a call needs only while it runs (gradient replays, ray
-// queries), kept for the next one: allocating and freeing it took longer than
-// many of these calls (64 K ray queries 2.0 ms with it, 0.4 without; the
-// gradient of a 512 x 512 texture 23 and 14 ms). Grow-only; what exceeds KEEP is
-// given back when the call ends. Used under the instance's iterationMutex, on
-// its stream.
-struct CallScratch {
-	static constexpr size_t KEEP = size_t(512) << 20;
-	char* device = nullptr;
-	size_t bytes = 0;
-	cudaError_t reserve(size_t need);
-	void trim();                   // after the call, with its stream idle
 	void release();
 };
 
