@@ -524,7 +524,7 @@ bool build_device_scene(MufflonInstance& inst, std::string& err) {
 	S.hasAlpha = hasAlpha ? 1 : 0;
 	S.sphereLights = numSphere64 > 0 ? 1 : 0;
 	S.tlasNodes = D.tlas.nodes; S.tlasPrimIds = D.tlas.primIds; S.tlasNumInternal = D.tlas.numInternal;
-	S.tlasWide = D.tlas.wnodes; S.tlasWidePrims = D.tlas.wprims; S.tlasNumWide = D.tlas.numWide;
+	S.tlasWide = D.tlas.wnodes; S.tlasNumWide = D.tlas.numWide;
 	S.materials = D.dMaterials; S.textures = D.dTextures;
 	S.lights = D.dLights; S.lightNodes = D.dLightNodes; S.lightPrimKeys = D.dLightKeys; S.lightPrimCodes = D.dLightCodes;
 	S.numLightPrims = numArea;

@@ -122,7 +122,6 @@ struct DScene {
 	const int32_t* tlasPrimIds;
 	int32_t tlasNumInternal;
 	const WideNode* tlasWide;
-	const int32_t* tlasWidePrims; // wide leaf slot -> instance id
 	int32_t tlasNumWide;
 	const DMaterial* materials;
 	const DTexture* textures;

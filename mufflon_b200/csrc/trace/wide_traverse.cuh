@@ -41,7 +41,7 @@ namespace mb {
 constexpr int WIDE_STACK = 64;
 
 // The traversal stack of one ray. The node group being visited lives in
-// registers (WideTracer::ngBase/ngMask, pgBase/pgHits); pushed groups
+// registers (WideTracerT::ngBase/ngMask, pgBase/pgHits); pushed groups
 // go to this per-thread array in local memory, which the L1 cache serves.
 // (Keeping the first 4, 8 or 16 entries in shared memory instead, thread-
 // interleaved, measured 5-7 % slower in the trace kernel on the B200.)
@@ -478,8 +478,6 @@ struct WideTracerT {
 
 	MBD const DLod& lod(const DScene& S) const { return S.lods[__ldg(S.instanceLod + inst)]; }
 };
-
-using WideTracer = WideTracerT<ALPHA_SCENE>;
 
 // Closest hit of a world-space ray whose origin is already offset.
 template < int AM = ALPHA_SCENE, class Stack, class C >
