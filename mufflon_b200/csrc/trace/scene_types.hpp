@@ -143,7 +143,7 @@ struct DScene {
 	int32_t hasAlpha;             // some material has an alpha texture
 	int32_t sphereLights;         // emissive spheres in the light list (their hit pdf needs the previous vertex)
 	// Traversal steps a ray may take (per traversal loop of the binary
-	// hierarchies, per ray of the 8-wide ones: WideTracerT::spend) before it is
+	// hierarchies, per ray of the 8-wide ones: WideTracerT::exceeded) before it is
 	// abandoned and counted as an error; MAX_TRAVERSAL_STEPS unless the renderer
 	// parameter "Traversal step limit" sets it.
 	int32_t maxSteps;
