@@ -2,13 +2,16 @@
 // Karras hierarchy of an LBVH build (the same tree whose collapsed form is
 // exported in the reference's BvhNode layout).
 //
-// The format follows the idea of Ylitie, Karras and Laine, "Efficient
-// Incoherent Ray Traversal on GPUs Through Compressed Wide BVHs" (HPG 2017):
-// child boxes are stored as 8-bit offsets on a per-node power-of-two grid,
-// internal children are stored contiguously, leaf primitives of a node are
-// stored contiguously, and children are placed in slots by direction octant so
-// that a ray visits them roughly near to far without sorting. The layout and
-// the conversion below are this project's own:
+// The format follows Ylitie, Karras and Laine, "Efficient Incoherent Ray
+// Traversal on GPUs Through Compressed Wide BVHs" (HPG 2017): child boxes are
+// stored as 8-bit offsets on a per-node power-of-two grid, internal children
+// are stored contiguously, leaf primitives of a node are stored contiguously,
+// and children are placed in slots by direction octant so that a ray visits
+// them roughly near to far without sorting. The meta byte (a unary count above
+// an offset, 24 + slot for internal children) and the way a ray turns it into
+// its hit masks and its octant's order (wide_node_test) are the paper's too.
+// The margin, the rounding, the leaf sizes and the conversion are this
+// project's own:
 //
 //   * 80-byte node, five 16-byte loads;
 //   * every quantised box contains its child's exact box with a margin of one
@@ -36,6 +39,10 @@ constexpr int WIDE_LEAF_MAX = 3;       // primitives per leaf in object hierarch
 // 1, 4 096 instances 720p 12.9 / 12.3 / 12.1 ms, plane 1.50 / 1.45 / 1.47 ms,
 // icosphere 1080p 2.89 / 2.85 / 2.90 ms; but the cut-outs' objects of up to two
 // dozen primitives, mostly one node each with leaves of three, 1.61 / 1.67 / 1.67.
+// The line at 64 keeps those and is no optimum for others: 300 instances of an
+// object of scattered triangles, quads and spheres, leaves of 3 / 2: 8
+// primitives 3.72 / 3.74 ms, 16 9.2 / 7.0, 24 7.9 / 6.8, 32 6.7 / 6.4, 48 7.2 /
+// 6.9, 64 6.6 / 6.4, 96 8.5 / 8.3, 128 8.0 / 7.3, 1 000 9.4 / 8.7.
 inline int wide_leaf_max(size_t n) { return n <= 64 ? WIDE_LEAF_MAX : 2; }
 constexpr int WIDE_TLAS_LEAF_MAX = 1;  // instances per leaf in the instance hierarchy
 

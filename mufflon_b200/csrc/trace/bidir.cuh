@@ -292,7 +292,9 @@ enum { BPTW_EXT0 = 0, BPTW_SH0 = 2, BPTW_WORK = 4 };
 // path tracer 748 / 765 / 764 and VCM 468 / 479 / 490 Mrays/s at 4 / 6 / 8;
 // 12 blocks (42 registers, more spills) fell back to 715 and 497.
 constexpr int BPTW_SHADE_BLOCKS = 8;
-// ... and the trace stage (5 and 6 measured alike; 8 was 6 % slower).
+// ... and the trace stage. 5 and 6 blocks, with voted steps (96 and 80
+// registers), 1080p icosphere: bidirectional path tracer 7.34 and 7.60 ms an
+// iteration, VCM 10.11 and 10.36.
 constexpr int BPTW_TRACE_BLOCKS = 5;
 // Resident blocks per SM of the connection kernels (k_bptw_connect,
 // k_vcmw_connect) and of VCM's merge kernel. Measured at 1080p (Mrays/s,

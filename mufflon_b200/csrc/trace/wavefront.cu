@@ -762,10 +762,11 @@ __global__ void __launch_bounds__(128, 8) k_shade(const SP sp, WfState W, int q,
 // of the loop traces at most one ray per lane (a shadow ray or the next
 // extension ray) in one traversal loop shared by the warp. A path's random
 // numbers, terms and their order are those of shade_vertex. It is bound by
-// instruction fetch (ncu: 9.4 of 15 cycles between issues). Running in each
-// pass the one state that most lanes wait in, as warp_step does, raised the
-// lanes per instruction from 2.7 to 5.8 but the time from 0.42 to 0.48 ms
-// (256 x 256 box): the shading code is fetched as often, for fewer paths.
+// instruction fetch (ncu, 256 x 256 box: 7 of 12 cycles between issues, at 4
+// lanes per instruction). Running in each pass the one state that most lanes
+// wait in, as warp_step does, doubled the lanes per instruction but took 0.48
+// instead of 0.42 ms (the same box, with 4 blocks an SM and 2.7 lanes): the
+// shading code is fetched as often, for fewer paths.
 template < int MINB, class SP, class C, int AM >
 __global__ void __launch_bounds__(128, MINB) k_tail(const SP sp, WfState W, int q, int bounce,
                                                     int workIdx, TraceCounters* counters, int neeCount, unsigned tailMax,
@@ -1179,6 +1180,9 @@ template < class SP > TraceKernel<SP> trace_kernel(int perSm, bool counting, boo
 // blocks. Tail of an iteration with 5 / 4 / 3 / 2 blocks: 256 x 256 box 0.307 /
 // 0.271 / 0.261 / 0.248 ms, 64 x 64 box 0.147 / 0.134 / 0.131 / 0.140, 1080p
 // icosphere 0.539 / 0.462 / 0.442 / 0.433, cutouts 0.182 / 0.161 / 0.149 / 0.147.
+// 3 rather than 2: the smallest images, whose iteration the tail is half of,
+// lose 3 % with 2 (0.247 and 0.254 ms), against 2 % gained at 256 x 256 (0.461
+// and 0.452) and nothing beyond the spread on the larger ones.
 constexpr int TAIL_BLOCKS = 3;
 
 template < class SP > struct TailKernel {

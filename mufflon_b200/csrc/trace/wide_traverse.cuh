@@ -17,16 +17,16 @@
 // the same arithmetic in every lane) and then that node's hit primitives.
 //
 // What bounds it: divergence and instruction issue (ncu, incoherent bounce of
-// the icosphere: 50 % of issue slots, 36 % of the ALU pipe, memory below 10 %
+// the icosphere: 54 % of issue slots, 41 % of the ALU pipe, memory below 10 %
 // of its peak; see warp_step), so the step is written for few
 // instructions and registers: box planes from biased bytes in packed
-// multiply-adds, hit masks by shifts of precomputed bytes,
-// reciprocals without special cases for boxes, one record per instance, no world-ray shear
-// constants, entering an instance in the step that visits its root. Against
-// a form with divisions, a subtraction per plane byte, out-of-line
-// instance transforms and the prepared world ray in registers (same box, per
-// iteration): trace stage of the 1080p icosphere 2.90 -> 2.12 ms, of 4 096
-// instances at 720p 15.4 -> 14.3 ms.
+// multiply-adds, hit masks by shifts of precomputed bytes, reciprocals without
+// special cases for boxes, one record per instance, no world-ray shear
+// constants, entering an instance in the step that visits its root. Against a
+// form with divisions, a subtraction per plane byte, out-of-line instance
+// transforms and the prepared world ray in registers (same box, per iteration,
+// both before the votes): trace stage of the 1080p icosphere 2.90 -> 2.12 ms,
+// of 4 096 instances at 720p 15.4 -> 14.3 ms.
 //
 // The box test cannot cull a box that contains a hit point (wide.hpp), so the
 // closest hit is the minimum of (world t, instance, primitive) over all
@@ -440,17 +440,18 @@ struct WideTracerT {
 	// three parts a pass ran the node test at 14 and the others at 2-5 lanes;
 	// without the votes the compiler besides threads a ray that entered an
 	// instance into a copy of the node test of its own, and the lanes drift
-	// apart.) ncu, incoherent bounces: 12.9 of 32 lanes per instruction against
-	// 9.0 (icosphere, 540p) and, with 38 % fewer instructions, against 5.6 to 9.9
-	// (4 096 instances, 360p) for steps without and with a meeting of the lanes
-	// between the parts. Weights: instances 3 and primitives 2 measured 10.3 ms
-	// of trace per 720p iteration of the instanced scene, 2 and 2 10.7, 1 and 1
-	// 11.7, 2 and 3 10.5, no votes 13.1; the icosphere is within 2 % for all.
+	// apart.) ncu, incoherent bounces: 12.7 of 32 lanes per instruction, 9.0
+	// before the votes (icosphere, 540p), and 14.2, 5.6 to 9.9 for steps without
+	// and with a meeting of the lanes between the parts (4 096 instances, 360p).
+	// Weights: instances 3 and primitives 2 measured 10.3 ms of trace per 720p
+	// iteration of the instanced scene, 2 and 2 10.7, 1 and 1 11.7, 2 and 3 10.5,
+	// no votes 13.1; the icosphere is within 2 % for all.
 	// With at most EACH rays left the warp runs all parts in every pass: few
 	// rays gain little from company, and a launch's last rays and a short queue
-	// wait for each pass (64 x 64 box 0.264 -> 0.246 ms an iteration, cut-outs
-	// 1.65 -> 1.56, bidirectional 1080p 7.43 -> 7.29; 4, 8, 14 and 22 rays: cut-outs
-	// 1.64, 1.61, 1.56, 1.53, 4 096 instances 12.3, 12.25, 12.2, 12.25).
+	// wait for each pass (against votes at any number, 64 x 64 box 0.264 -> 0.246
+	// ms an iteration, cut-outs 1.65 -> 1.56, bidirectional 1080p 7.43 -> 7.29).
+	// 14, 16 and 22 rays: cut-outs 1.600, 1.594, 1.567 ms, 4 096 instances 12.24,
+	// 12.24, 12.30, the other scenes within their spread.
 	template < class Stack, class C >
 	MBD bool warp_step(const DScene& S, C& cnt, Stack& stack, bool active) {
 		constexpr int INSTANCE_WEIGHT = 3, PRIM_WEIGHT = 2, EACH = 16;
