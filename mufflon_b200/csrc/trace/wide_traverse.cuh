@@ -126,6 +126,16 @@ static __device__ __noinline__ PrimHit other_prim_test(const DLod* l, f3 o, f3 d
 	h.hit = prim_test(*l, other_ray(*l, o, d, p), 0, p, h.t, h.uv);
 	return h;
 }
+// The alpha test's scene in kernels that were compiled with it. Whether it
+// applies is the kernel's to say, not S.hasAlpha's: a batch with cut-outs in
+// one job's scene runs such kernels over all of them, and the materials of the
+// others name no alpha texture.
+MBD AlphaCtx alpha_all(const DScene& S) {
+	AlphaCtx a;
+	a.materials = S.materials;
+	a.textures = S.textures;
+	return a;
+}
 static __device__ __noinline__ PrimHit other_prim_test_alpha(const DLod* l, f3 o, f3 d, int p, AlphaCtx alpha) {
 	PrimHit h;
 	h.hit = prim_test(*l, other_ray(*l, o, d, p), 0, p, h.t, h.uv, alpha);
@@ -392,9 +402,9 @@ struct WideTracerT {
 		bool hit;
 		if(__float_as_int(b.w) == SOUP_TRIANGLE) {
 			hit = tri_test(o, int(axes & 3u), int(axes >> 2 & 3u), int(axes >> 4), Sx, Sy, Sz, f4to3(a), f4to3(b), f4to3(c), to, uv) && to > 0.0f;
-			if(ALPHA && hit) hit = !alpha_cuts_triangle(alpha_ctx(S), lod(S), p, uv);
+			if(ALPHA && hit) hit = !alpha_cuts_triangle(alpha_all(S), lod(S), p, uv);
 		} else {
-			const PrimHit ph = ALPHA ? other_prim_test_alpha(&lod(S), o, d, p, alpha_ctx(S)) : other_prim_test(&lod(S), o, d, p);
+			const PrimHit ph = ALPHA ? other_prim_test_alpha(&lod(S), o, d, p, alpha_all(S)) : other_prim_test(&lod(S), o, d, p);
 			hit = ph.hit; to = ph.t; uv = ph.uv;
 		}
 		if(hit) {

@@ -87,6 +87,30 @@ def test_batch_equals_single_job_render(worlds):
     assert np.array_equal(imgs[0], ref)
 
 
+@pytest.mark.parametrize("order", [(0, 1, 2), (2, 1, 0)])
+def test_cutouts_beside_scenes_without(order):
+    """One job's scene has alpha textures, the others' have not: triangles, quads and spheres of both."""
+    specs = [scenes.cornell_box(3, 40, 32), scenes.alpha_cutouts(4, 36, 44), scenes.emissive_panels(2, width=30, height=38, emissive_spheres=2)]
+    instances = [bindings.DllInterface() for _ in specs]
+    try:
+        for d, spec in zip(instances, specs):
+            bindings.load_scene_spec(d, spec)
+            assert d.render_enable_renderer(0, 0)
+            d.render_enable_render_target("Radiance", False)
+            assert d.renderer_set_parameter_int("Seed", 5)
+            assert d.renderer_set_parameter_int("Max. path length", 6)
+        imgs, _, _, _ = bindings.render_batch([dict(instance=instances[k], spp=3, max_path=6, seed=5) for k in order])
+        for img, k in zip(imgs, order):
+            instances[k].render_reset()
+            for _ in range(3):
+                instances[k].render_iterate()
+            assert np.array_equal(img, instances[k].get_target_image("Radiance")), specs[k].name
+            assert img.mean() > 0.0
+    finally:
+        for d in instances:
+            d.close()
+
+
 def test_batch_rejects_bad_jobs(worlds):
     d, _ = worlds["cornell"]
     with pytest.raises(bindings.MufflonError):
